@@ -108,10 +108,11 @@ def _device() -> AudioDevice:
 
 
 class _Handle:
-    """An object of the C API, destroyed with its owner."""
+    """An object of the C API, destroyed with its owner and before the device it lives on."""
 
     def __init__(self, create, destroy, *args):
         self.lib = L.load()
+        self.device = _device()
         self._destroy = getattr(self.lib, destroy)
         self.h = ctypes.c_void_p()
         _ok(getattr(self.lib, create)(*args, ctypes.byref(self.h)))
