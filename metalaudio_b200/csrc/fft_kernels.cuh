@@ -869,6 +869,13 @@ inline bool istft_fast_ok(const C2RParams& p) {
     }
 }
 
+// The part of a sample pair that lies before the end of the output row, `left` samples away: the last
+// frame of a convolution reaches up to N - 1 samples past it.
+MA_HD void store_pair_before(float* o, float2 r, int64_t left) {
+    if (left >= 2) *reinterpret_cast<float2*>(o) = r;
+    else if (left == 1) *o = r.x;
+}
+
 template <int M, int LAYOUT, int OVT, class Cta>
 MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
     using P = FftPlan<M>;
@@ -1048,7 +1055,7 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
                                 r2.y = r2.y / window_sum_at(p.window, o + 1, N, hop, F, p.floor);
                             }
                         }
-                        *reinterpret_cast<float2*>(out + i0) = r2;
+                        store_pair_before(out + i0, r2, p.out_len - (start + i0));
                     }
                     if (q >= HR) racc[q - HR] = acc;
                 }
@@ -1080,7 +1087,7 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
                             r2.y = acc.y / window_sum_at(p.window, o + 1, N, hop, F, p.floor);
                         }
                     }
-                    *reinterpret_cast<float2*>(out + i0) = r2;
+                    store_pair_before(out + i0, r2, p.out_len - (start + i0));
                 }
             } else {
                 *slot = acc;

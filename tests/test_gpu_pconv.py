@@ -164,6 +164,30 @@ def test_streaming_step_with_forced_partition_splits(device, lib, splits):
         assert o64.rel_rms(y[i], o64.convolve_full(x[i], h)[:length]) <= TOL
 
 
+@pytest.mark.parametrize("block,taps,length", [(128, 1001, 5000), (512, 1025, 4096), (32, 65, 1000), (1024, 4097, 20480)])
+def test_whole_signal_writes_only_its_rows(device, lib, block, taps, length):
+    """Rows packed at exactly len + taps - 1 samples (an even count: the paired plans' overlap-add):
+    the samples behind every row belong to the next channel, those behind the last one to nobody."""
+    from metalaudio_b200 import Tensor
+    channels = 3
+    rng = np.random.default_rng(block)
+    h = (rng.standard_normal(taps) / np.sqrt(taps)).astype(np.float32)
+    x = rng.standard_normal((channels, length)).astype(np.float32)
+    full = length + taps - 1
+    c = conv(device, block, channels=channels)
+    c.setKernel(h)
+    guard = 4 * block
+    tin = Tensor(device, x.shape); tin.copy(x)
+    tout = Tensor(device, (channels * full + guard,)); tout.copy(np.full(channels * full + guard, 7.0, np.float32))
+    assert lib.ma_pconv_reserve(c._h, length) == 0
+    assert lib.ma_pconv_process_dev(c._h, ctypes.c_void_p(tin.pointer), length, length, ctypes.c_void_p(tout.pointer), full) == 0
+    device.synchronize()
+    y = tout.toArray()
+    assert np.all(y[channels * full:] == 7.0)
+    for i in range(channels):
+        assert o64.rel_rms(y[i * full:(i + 1) * full], o64.convolve_full(x[i], h)) <= TOL
+
+
 def test_config3_scaled(device):
     """Configuration 3 at reduced channel count / length: one shared exponentially decaying
     noise IR, block 256, float64 oracle plus exact dot-product spot checks."""

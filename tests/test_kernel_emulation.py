@@ -117,6 +117,31 @@ def test_stft_istft(emul, n, hop, length, chunks, kind):
     assert o64.rel_rms(y[:, msk], yref[:, msk]) <= 1e-5
 
 
+@pytest.mark.parametrize("n,cut", [(256, 1), (256, 130), (256, 200), (1024, 777), (4096, 4000)])
+@pytest.mark.parametrize("hop_div", [2, 4])
+def test_overlap_add_stops_at_the_end_of_the_output_row(emul, n, cut, hop_div):
+    """The convolution's overlap-add ends at len + taps - 1 samples, anywhere inside the last frame:
+    nothing behind the row may be touched, on the paired plans' kernels either."""
+    hop, f, signals = n // hop_div, 5, 2
+    out_len = (f - 1) * hop + n - cut
+    stride = out_len + 2 * n + (out_len & 1)
+    rng = np.random.default_rng(n + cut)
+    x = rng.standard_normal((signals, f, n)).astype(np.float32)
+    spec = np.ascontiguousarray(np.fft.rfft(x, axis=-1).astype(np.complex64)).view(np.float32)
+    y = np.full((signals, stride), 7.0, np.float32)
+    w = np.ones(n, np.float32)
+    rc = emul.emul_istft(n, hop, fp(spec), None, f * (n // 2 + 1), n // 2 + 1, f, signals, 0, fp(w), 1e-8, fp(y), stride,
+                         out_len, 2, 2)
+    assert rc == 1
+    assert np.all(y[:, out_len:] == 7.0)
+    full = (f - 1) * hop + n
+    ref, ws = np.zeros((signals, full)), np.zeros(full)
+    for k in range(f):
+        ref[:, k * hop:k * hop + n] += x[:, k]
+        ws[k * hop:k * hop + n] += 1.0
+    assert o64.rel_rms(y[:, :out_len], (ref / ws)[:, :out_len]) <= 1e-6
+
+
 @pytest.mark.parametrize("partitions", [1, 4, 5, 8, 15, 16, 17, 20, 24, 31, 32, 33, 64, 100, 512])
 @pytest.mark.parametrize("blocks", [1, 3, 63, 64, 65, 200])
 def test_tiled_multiply_accumulate_row_schedule(emul, partitions, blocks):
