@@ -39,9 +39,19 @@ struct ma_pconv {
     int splits = 1;              // partition splits of the streaming step
     float2* d_partial = nullptr; // [splits][C][B]
     int64_t reserved_len = 0;
-    int64_t reserved_blocks = 0;
     float2* d_timeline = nullptr;
     float2* d_y = nullptr;
+    // Whole-signal calls that start on a clear delay line need not keep the caller's block size: they run on
+    // a coarser partition of the same taps (whole_block), built by ma_pconv_reserve.  Where the caller's own
+    // block is the better one, w_plan and d_hw are plan and d_h.
+    float* d_taps = nullptr;      // [n_irs][taps_stride], kept from set_kernels until the coarse spectra exist
+    int64_t taps_stride = 0;
+    int w_block = 0, w_partitions = 0;
+    ma_fft_plan* w_plan = nullptr;
+    float2* d_hw = nullptr;
+    int64_t w_stride = 0;         // float2 per channel of the coarse timeline
+    bool clear = true;            // every delay-line spectrum a later call can reach, and the tail, are zero
+    bool prefix_clear = false;    // the w_partitions - 1 rows in front of each channel's coarse timeline are zero
 };
 
 namespace ma {
@@ -353,7 +363,7 @@ constexpr int kTwoLevelFrom = 2048;
 static ma_status launch_mac_tiled(ma_pconv* pc, const MacParams& q, int channels, int64_t t_count, int64_t tl_len) {
     constexpr int TT = 16;
     ma_context* ctx = pc->ctx;
-    const int bin_tiles = pc->block >> 5;
+    const int bin_tiles = q.block >> 5;
     const int64_t t_ctas = (t_count + 4 * TT - 1) / (4 * TT);
     int64_t done = 0;
     while (done < t_ctas) {  // grid.y limit
@@ -362,10 +372,10 @@ static ma_status launch_mac_tiled(ma_pconv* pc, const MacParams& q, int channels
         MacParams qq = q;
         const int64_t t_first = done * 4 * TT;
         qq.out = q.out + t_first * q.out_t_stride;
-        qq.x = q.x + t_first * pc->block;  // shifts the timeline origin by t_first rows
+        qq.x = q.x + t_first * q.block;  // shifts the timeline origin by t_first rows
         dim3 grid((unsigned)(bin_tiles * channels), (unsigned)ny, 1);
         // Blocked summation once a running sum would cover more than kTwoLevelFrom partitions.
-        if (pc->partitions >= kTwoLevelFrom)
+        if (q.partitions >= kTwoLevelFrom)
             pconv_mac_tiled_kernel<TT, true><<<grid, 128, 0, ctx->stream>>>(qq, (int)(t_count - t_first), tl_len - t_first);
         else
             pconv_mac_tiled_kernel<TT, false><<<grid, 128, 0, ctx->stream>>>(qq, (int)(t_count - t_first), tl_len - t_first);
@@ -413,7 +423,7 @@ static ma_status launch_mac_t(ma_context* ctx, const MacParams& q, int chan_tile
 }
 
 static ma_status launch_mac(ma_pconv* pc, MacParams q, int channels, bool stream, int64_t t_count) {
-    const int B = pc->block;
+    const int B = q.block;
     const int vec = B >= 2 ? 2 : 1;
     const int bp = B / vec;  // threads per spectrum
     q.bpt = bp < kMacThreads ? bp : kMacThreads;
@@ -491,16 +501,87 @@ __global__ void pconv_history_kernel(float2* __restrict__ ring, float2* __restri
     }
 }
 
+// Largest block of the whole-signal calls: 4096-point transforms, the longest with the paired plans.
+constexpr int kWholeBlock = 2048;
+constexpr int kWholePartitions = 8;
+
 static void free_signal_buffers(ma_pconv* pc) {
     if (pc->d_timeline) (void)cudaFree(pc->d_timeline);
     if (pc->d_y) (void)cudaFree(pc->d_y);
     pc->d_timeline = nullptr;
     pc->d_y = nullptr;
     pc->reserved_len = 0;
-    pc->reserved_blocks = 0;
+    pc->prefix_clear = false;
+}
+
+// Partition spectra: the taps are the "signals", partitions the "frames" at hop `block`, each
+// frame's samples beyond `block` (and beyond the end of the response) read as zero.
+static ma_status partition_spectra(ma_pconv* pc, ma_fft_plan* plan, int block, int partitions, float2* h) {
+    R2CParams p{};
+    p.in = pc->d_taps;
+    p.signal_stride = pc->taps_stride;
+    p.frames_per_signal = partitions;
+    p.total_frames = (int64_t)partitions * pc->n_irs;
+    p.signal_len = pc->taps;
+    p.hop = block;
+    p.frame_valid = block;
+    p.out_a = reinterpret_cast<float*>(h);
+    p.out_signal_stride = (int64_t)partitions * block;
+    p.out_frame_stride = block;
+    p.layout = LAYOUT_HALF_PACKED;
+    p.mag_kind = MAG_NONE;
+    return launch_r2c_small(plan, p);
+}
+
+static void free_coarse(ma_pconv* pc) {
+    if (pc->w_plan && pc->w_plan != pc->plan) (void)ma_fft_plan_destroy(pc->w_plan);
+    if (pc->d_hw && pc->d_hw != pc->d_h) (void)cudaFree(pc->d_hw);
+    pc->w_plan = nullptr;
+    pc->d_hw = nullptr;
+}
+
+// Block size of whole-signal calls.  The multiply-accumulate costs one complex product per output bin and
+// partition, i.e. it shrinks with the number of partitions, while the transforms' cost per sample hardly
+// depends on their length up to 4096 points.  The shorter sums also round less, which pays for the longer
+// transforms' rounding as long as there are sums to shorten: at least kWholePartitions partitions stay.
+// Measured, 512 channels x 2^20 samples, 131072 taps, block 256: 512 partitions 64.2 ms, error 4.4e-7; 64 partitions
+// of 2048 samples 15.2 ms (10.8 ms with the paired plans' block transforms), error 2.9e-7.
+static int whole_block(int block, int64_t taps) {
+    int b = block;
+    while (b < kWholeBlock && 2 * (int64_t)b * kWholePartitions <= taps) b *= 2;
+    return b;
+}
+
+// Plan and partition spectra of the whole-signal calls.  Without the memory for them the caller's own
+// block size serves those calls too.
+static void build_coarse(ma_pconv* pc) {
+    pc->w_block = whole_block(pc->block, pc->taps);
+    pc->w_partitions = (int)((pc->taps + pc->w_block - 1) / pc->w_block);
+    if (pc->w_block != pc->block) {
+        ma_context* ctx = pc->ctx;
+        ma_status st = ma_fft_plan_create(ctx, 2 * pc->w_block, nullptr, pc->w_block, &pc->w_plan);
+        if (st == MA_OK) {
+            cudaError_t e = cudaMalloc((void**)&pc->d_hw, sizeof(float2) * (size_t)pc->w_partitions * pc->w_block * (size_t)pc->n_irs);
+            if (e != cudaSuccess) st = cuda_fail(e);
+        }
+        if (st == MA_OK) st = partition_spectra(pc, pc->w_plan, pc->w_block, pc->w_partitions, pc->d_hw);
+        if (st == MA_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) st = MA_ERR_CUDA;
+        if (st != MA_OK) free_coarse(pc);
+    }
+    if (pc->w_plan == nullptr) {
+        pc->w_block = pc->block;
+        pc->w_partitions = pc->partitions;
+        pc->w_plan = pc->plan;
+        pc->d_hw = pc->d_h;
+    }
+    (void)cudaFree(pc->d_taps);
+    pc->d_taps = nullptr;
 }
 
 static void free_kernel_buffers(ma_pconv* pc) {
+    free_coarse(pc);
+    if (pc->d_taps) (void)cudaFree(pc->d_taps);
+    pc->d_taps = nullptr;
     if (pc->d_h) (void)cudaFree(pc->d_h);
     if (pc->d_ch2ir) (void)cudaFree(pc->d_ch2ir);
     if (pc->d_ring) (void)cudaFree(pc->d_ring);
@@ -621,30 +702,15 @@ ma_status ma_pconv_set_kernels(ma_pconv* pc, const float* irs, int64_t taps, int
         e = cudaMalloc((void**)&pc->d_partial, sizeof(float2) * (size_t)pc->splits * (size_t)C * B);
     if (e != cudaSuccess) st = cuda_fail(e);
     if (st == MA_OK) st = copy_h2d(ctx, pc->d_ch2ir, map.data(), sizeof(int32_t) * (size_t)C);
-    // Partition spectra: the taps are the "signals", partitions the "frames" at hop B, each
-    // frame's samples beyond B (and beyond the end of the IR) read as zero.
-    float* d_taps = nullptr;
-    const int64_t tstride = taps + (taps & 1);
-    if (st == MA_OK) st = temp_alloc(ctx, sizeof(float) * (size_t)(tstride * n_irs), (void**)&d_taps);
-    for (int i = 0; i < n_irs && st == MA_OK; ++i)
-        st = copy_h2d(ctx, d_taps + (int64_t)i * tstride, irs + (int64_t)i * taps, sizeof(float) * (size_t)taps);
+    const int64_t tstride = (taps + 3) & ~(int64_t)3;
+    pc->taps_stride = tstride;
     if (st == MA_OK) {
-        R2CParams p{};
-        p.in = d_taps;
-        p.signal_stride = tstride;
-        p.frames_per_signal = P;
-        p.total_frames = (int64_t)P * n_irs;
-        p.signal_len = taps;
-        p.hop = B;
-        p.frame_valid = B;
-        p.out_a = reinterpret_cast<float*>(pc->d_h);
-        p.out_signal_stride = (int64_t)P * B;
-        p.out_frame_stride = B;
-        p.layout = LAYOUT_HALF_PACKED;
-        p.mag_kind = MAG_NONE;
-        st = launch_r2c_small(pc->plan, p);
+        e = cudaMalloc((void**)&pc->d_taps, sizeof(float) * (size_t)(tstride * n_irs));
+        if (e != cudaSuccess) st = cuda_fail(e);
     }
-    temp_free(ctx, d_taps);
+    for (int i = 0; i < n_irs && st == MA_OK; ++i)
+        st = copy_h2d(ctx, pc->d_taps + (int64_t)i * tstride, irs + (int64_t)i * taps, sizeof(float) * (size_t)taps);
+    if (st == MA_OK) st = partition_spectra(pc, pc->plan, B, P, pc->d_h);
     if (st == MA_OK) st = ma_pconv_reset(pc);
     if (st == MA_OK) {
         cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
@@ -689,6 +755,7 @@ ma_status ma_pconv_reset(ma_pconv* pc) {
     MA_CUDA(cudaMemsetAsync(pc->d_ring, 0, ring_bytes, pc->ctx->stream));
     MA_CUDA(cudaMemsetAsync(pc->d_tail, 0, sizeof(float) * (size_t)pc->channels * pc->block, pc->ctx->stream));
     pc->write_index = 0;
+    pc->clear = true;
     return MA_OK;
 }
 
@@ -701,42 +768,65 @@ ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len) {
     if (max_len <= pc->reserved_len) return MA_OK;
     int64_t full;
     if (__builtin_add_overflow(max_len, pc->taps - 1, &full)) return MA_ERR_OUTPUT_OVERFLOW;
-    const int64_t blocks = (full + pc->block - 1) / pc->block;
     MA_CUDA(cudaStreamSynchronize(ctx->stream));
     free_signal_buffers(pc);
-    const size_t row = (size_t)pc->block * sizeof(float2);
-    const size_t tl_bytes = (size_t)pc->channels * (size_t)(pc->partitions - 1 + blocks) * row;
-    const size_t y_bytes = (size_t)pc->channels * (size_t)blocks * row;
-    cudaError_t e = cudaMalloc((void**)&pc->d_timeline, tl_bytes ? tl_bytes : 16);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&pc->d_y, y_bytes ? y_bytes : 16);
+    if (pc->w_plan == nullptr) build_coarse(pc);
+    // both partitions share the buffers: the caller's block size serves calls that continue a stream
+    auto blocks = [&](int b) { return (full + b - 1) / b; };
+    const int64_t own_row = (pc->partitions - 1 + blocks(pc->block)) * pc->block;
+    pc->w_stride = (pc->w_partitions - 1 + blocks(pc->w_block)) * pc->w_block;
+    const int64_t tl_row = own_row > pc->w_stride ? own_row : pc->w_stride;
+    const int64_t own_y = blocks(pc->block) * pc->block, w_y = blocks(pc->w_block) * pc->w_block;
+    cudaError_t e = cudaMalloc((void**)&pc->d_timeline, sizeof(float2) * (size_t)pc->channels * (size_t)tl_row);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void**)&pc->d_y, sizeof(float2) * (size_t)pc->channels * (size_t)(own_y > w_y ? own_y : w_y));
     if (e != cudaSuccess) {
         ma_status st = cuda_fail(e);
         free_signal_buffers(pc);
         return st;
     }
     pc->reserved_len = max_len;
-    pc->reserved_blocks = blocks;
     return MA_OK;
 }
 
 }  // extern "C"
 
+// Once per whole-signal call, before its channel ranges: the rows in front of the coarse timeline.
+static ma_status open_whole(ma_pconv* pc) {
+    if (!pc->clear) pc->prefix_clear = false;  // this call lays the buffer out by the caller's block size
+    if (!pc->clear || pc->prefix_clear || pc->w_partitions == 1) return MA_OK;
+    MA_CUDA(cudaMemset2DAsync(pc->d_timeline, sizeof(float2) * (size_t)pc->w_stride, 0,
+                              sizeof(float2) * (size_t)(pc->w_partitions - 1) * (size_t)pc->w_block, (size_t)pc->channels,
+                              pc->ctx->stream));
+    pc->prefix_clear = true;
+    return MA_OK;
+}
+
+// ... and after them.  A call pushes ceil((len + taps - 1)/B) >= ceil(len/B) + P - 1 blocks, so the only
+// spectrum of its input that can still be in the delay line is in the slot the next block overwrites.
+static void close_whole(ma_pconv* pc) {
+    pc->write_index = 0;
+    pc->clear = true;
+}
+
 // Whole-signal convolution of channels [c0, c0 + nc) (nc a multiple of the IR-sharing group): `in`
 // and `out` point at channel c0's rows.  Every buffer of the object is per channel, so a range runs
-// on its own slices; the delay-line position is reset by the caller once all ranges are queued.
+// on its own slices between open_whole and close_whole.
 static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, int64_t len, int64_t in_stride,
                                float* out, int64_t out_stride, int64_t full) {
     ma_context* ctx = pc->ctx;
-    const int B = pc->block, P = pc->partitions;
+    const bool coarse = pc->clear;
+    ma_fft_plan* plan = coarse ? pc->w_plan : pc->plan;
+    const int B = coarse ? pc->w_block : pc->block, P = coarse ? pc->w_partitions : pc->partitions;
     const int64_t T = (full + B - 1) / B;
     const int64_t tl_len = (int64_t)P - 1 + T;
-    const int64_t tl_stride = tl_len * B;
-    float2* ring = pc->d_ring + (int64_t)c0 * P * B;
+    const int64_t tl_stride = coarse ? pc->w_stride : tl_len * B;
+    float2* ring = pc->d_ring + (int64_t)c0 * pc->partitions * pc->block;
     float2* timeline = pc->d_timeline + (int64_t)c0 * tl_stride;
     float2* y = pc->d_y + (int64_t)c0 * T * B;
 
-    // 1. history -> timeline prefix
-    if (P > 1) {
+    // 1. history -> timeline prefix (a clear delay line: zeros since open_whole)
+    if (P > 1 && !coarse) {
         const int64_t total = (int64_t)nc * (P - 1) * B;
         int grid = (int)((total + 255) / 256 < (int64_t)ctx->sm_count * 8 ? (total + 255) / 256 : (int64_t)ctx->sm_count * 8);
         pconv_history_kernel<<<grid, 256, 0, ctx->stream>>>(ring, timeline, tl_stride, P, B, pc->write_index, 0, 1, nc);
@@ -757,14 +847,14 @@ static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, in
         p.out_frame_stride = B;
         p.layout = LAYOUT_HALF_PACKED;
         p.mag_kind = MAG_NONE;
-        MA_TRY(launch_r2c_small(pc->plan, p));
+        MA_TRY(launch_r2c_small(plan, p));
     }
     // 3. delay-line multiply-accumulate for every (channel, block)
     {
         MacParams q{};
         q.x = timeline;
         q.x_chan_stride = tl_stride;
-        q.h = pc->d_h;
+        q.h = coarse ? pc->d_hw : pc->d_h;
         q.ch2ir = pc->d_ch2ir + c0;
         q.out = y;
         q.out_split_stride = 0;
@@ -794,10 +884,10 @@ static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, in
         p.out_signal_stride = out_stride;
         p.out_len = full;
         p.floor = -1.0f;
-        MA_TRY(launch_istft_small(pc->plan, p));
+        MA_TRY(launch_istft_small(plan, p));
     }
-    // 5. the last P block spectra become the delay line
-    {
+    // 5. the last P block spectra become the delay line (clear before the call: it stays clear, see close_whole)
+    if (!coarse) {
         const int64_t total = (int64_t)nc * P * B;
         int grid = (int)((total + 255) / 256 < (int64_t)ctx->sm_count * 8 ? (total + 255) / 256 : (int64_t)ctx->sm_count * 8);
         pconv_history_kernel<<<grid, 256, 0, ctx->stream>>>(ring, timeline, tl_stride, P, B, 0, T - 1, 0, nc);
@@ -822,8 +912,9 @@ ma_status ma_pconv_process_dev(ma_pconv* pc, const float* in, int64_t len, int64
     if (__builtin_add_overflow(len, pc->taps - 1, &full)) return MA_ERR_OUTPUT_OVERFLOW;
     if (len > pc->reserved_len) return MA_ERR_INVALID_ARGUMENT;
     if (pc->channels > 1 && (in_stride < len || out_stride < full)) return MA_ERR_INVALID_ARGUMENT;
+    MA_TRY(open_whole(pc));
     MA_TRY(process_range(pc, 0, pc->channels, in, len, in_stride, out, out_stride, full));
-    pc->write_index = 0;
+    close_whole(pc);
     return MA_OK;
 }
 
@@ -848,6 +939,7 @@ ma_status ma_pconv_process_host(ma_pconv* pc, const float* in, int64_t len, int6
     const int group = pc->share;  // channels that must stay together (they share one impulse response)
     const size_t in_row = round256(sizeof(float) * (size_t)len), out_row = round256(sizeof(float) * (size_t)full);
     const bool pinned = is_pinned(in) && is_pinned(out);
+    MA_TRY(open_whole(pc));
     Pipe pp;
     MA_TRY(pipe_open(pp, ctx, pinned, C / group, (in_row + out_row) * (size_t)group, 0));
     const int64_t step = pp.chunk * group;
@@ -868,7 +960,7 @@ ma_status ma_pconv_process_host(ma_pconv* pc, const float* in, int64_t len, int6
         pp.after_copy_out(i);
     }
     const ma_status st = pp.finish();
-    if (st == MA_OK) pc->write_index = 0;
+    if (st == MA_OK) close_whole(pc);
     return st;
 }
 
@@ -883,6 +975,7 @@ ma_status ma_pconv_step_dev(ma_pconv* pc, const float* in_block, int64_t in_stri
     if (C > 1 && (in_stride < B || out_stride < B)) return MA_ERR_INVALID_ARGUMENT;
     if (pc->write_index < 0 || pc->write_index >= P) return MA_ERR_INVALID_PARTITION_STATE;
     const int w = pc->write_index;
+    pc->clear = false;
     // The three kernels are chained by programmatic dependent launch: this step's r2c may run
     // beside the previous step's c2r (see fft_small.cu).  That is only sound when the kernel right
     // before this r2c on the stream is that c2r and the two share no data: r2c reads its input

@@ -188,6 +188,49 @@ def test_whole_signal_writes_only_its_rows(device, lib, block, taps, length):
         assert o64.rel_rms(y[i * full:(i + 1) * full], o64.convolve_full(x[i], h)) <= TOL
 
 
+@pytest.mark.parametrize("block,taps", [(64, 1023), (64, 1024), (128, 2048), (64, 40001), (256, 33000), (2048, 40000)])
+def test_whole_signal_after_steps_and_back(device, lib, block, taps):
+    """Whole-signal calls on a clear delay line run on a coarser partition (from 16 partitions up); a call that
+    follows streaming steps continues with their history on the caller's block size, and the calls and
+    steps after it start clear again."""
+    from metalaudio_b200 import Tensor
+    channels, steps, length = 2, 3, 5000
+    rng = np.random.default_rng(taps)
+    h = (rng.standard_normal(taps) / np.sqrt(taps)).astype(np.float32)
+    x = rng.standard_normal((channels, steps * block + length)).astype(np.float32)
+    c = conv(device, block, channels=channels)
+    c.setKernel(h)
+    tail = np.ascontiguousarray(x[:, steps * block:])
+    ref = np.stack([o64.convolve_full(tail[i], h) for i in range(channels)])
+    tin = Tensor(device, x.shape); tin.copy(x)
+    tout = Tensor(device, (channels, block))
+
+    def step(t):
+        assert lib.ma_pconv_step_dev(c._h, ctypes.c_void_p(tin.pointer + 4 * t * block), x.shape[1],
+                                     ctypes.c_void_p(tout.pointer), block) == 0
+        device.synchronize()
+        return tout.toArray()
+
+    assert o64.rel_rms(c.process(tail), ref) <= TOL           # clear
+    for t in range(steps):
+        y = step(t)                                           # the call before left nothing behind
+    want = np.stack([o64.convolve_full(x[i, :steps * block], h)[(steps - 1) * block:steps * block] for i in range(channels)])
+    assert o64.rel_rms(y, want) <= TOL
+    # continues the stream: the block products of the steps' input reach into the call (all but the kept tail)
+    z = c.process(tail)
+    port = rp.PartitionedConvolution(block)
+    for i in range(channels):
+        port.set_kernel(h)
+        for t in range(steps):
+            padded = np.concatenate([x[i, t * block:(t + 1) * block], np.zeros(block, np.float32)])
+            port.ring[port.write_index] = np.fft.fft(padded).astype(np.complex64)
+            port.write_index = (port.write_index + 1) % port.partitions
+        assert o64.rel_rms(z[i], port.process(tail[i])) <= TOL
+    assert o64.rel_rms(c.process(tail), ref) <= TOL           # clear again
+    y = step(0)
+    assert o64.rel_rms(y, np.stack([o64.convolve_full(x[i, :block], h)[:block] for i in range(channels)])) <= TOL
+
+
 def test_config3_scaled(device):
     """Configuration 3 at reduced channel count / length: one shared exponentially decaying
     noise IR, block 256, float64 oracle plus exact dot-product spot checks."""
