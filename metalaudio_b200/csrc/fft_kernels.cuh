@@ -160,7 +160,10 @@ MA_HD void r2c_store_pair(const R2CParams& p, int64_t g, int64_t half_off, int k
 
 // ALIGNED: every frame start is 8-byte aligned and no zero padding is requested, so
 // sample pairs are fetched with one float2 load.  Otherwise scalar guarded loads.
-template <int M, bool ALIGNED, int LAYOUT, int MAGK, class Cta>
+// HALF: zero-padded blocks (frame_valid = M, the convolution's input), no window.  Only the first half
+// of a frame is staged or loaded, up to the end of the signal: whole 16-byte groups by the bulk copy,
+// what is left of a ragged end by guarded loads.
+template <int M, bool ALIGNED, int LAYOUT, int MAGK, class Cta, bool HALF = false>
 MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
     using P = FftPlan<M>;
     using S = CtaShape<M>;
@@ -172,7 +175,7 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
     int parity = 0;
 
     float2 wreg[R];
-    if (p.window != nullptr) {
+    if (!HALF && p.window != nullptr) {
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int n = t + q * T;
@@ -186,8 +189,11 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
     // Kernels with the layout fixed at compile time keep their twiddles in registers and have the
     // whole next frame staged by one bulk asynchronous copy (TMA unit).  (Per-thread 8-byte
     // asynchronous copies were tried instead: they cost more load/store-pipe wavefronts than they hide.)
-    constexpr bool TWALU = ALIGNED && LAYOUT >= 0 && plan_pairable<M>();
-    constexpr bool BULK = TWALU;
+    constexpr bool BULK = ALIGNED && LAYOUT >= 0 && plan_pairable<M>();
+    // The convolution's transforms (HALF) read the exact twiddles from the tables instead: a power chain
+    // multiplies the rounding of its base by the power, which there more than doubled the error of the whole
+    // convolution (2.0e-7 -> 4.9e-7 relative; 1.38 instead of 1.60 ms per 512 channels of 512 blocks).
+    constexpr bool TWALU = BULK && !HALF;
     float2 twb[tw_base_count<P>()];
     float2 wherm[R / 2 + 1];
     (void)wherm;
@@ -213,11 +219,20 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
     uint64_t* bar = reinterpret_cast<uint64_t*>(stage + S::STAGE) + 2 * slot;
     const bool bulk = BULK && p.bulk_ok != 0;
     uint32_t phase = 0;
+    // samples of frame f_ that exist (HALF); the bulk copy brings the whole groups of four among them
+    auto half_valid = [&](int64_t f_) {
+        const int64_t left = p.signal_len - f_ * (int64_t)p.hop;
+        return left >= M ? M : (left > 0 ? (int)left : 0);
+    };
+    auto start_copy = [&](int64_t s_, int64_t f_) {  // called by thread 0 of the slot
+        const uint32_t floats = HALF ? (uint32_t)(half_valid(f_) & ~3) : (uint32_t)N;
+        if (!HALF || floats > 0)
+            cta.bulk_copy(stage_slot, p.in + s_ * p.signal_stride + f_ * (int64_t)p.hop, floats * (uint32_t)sizeof(float), bar);
+    };
     if (bulk) {
         if (t == 0) cta.bulk_init(bar);
         cta.sync();
-        if (t == 0 && g < p.total_frames)
-            cta.bulk_copy(stage_slot, p.in + s * p.signal_stride + f * (int64_t)p.hop, N * (uint32_t)sizeof(float), bar);
+        if (t == 0 && g < p.total_frames) start_copy(s, f);
     }
     for (int64_t base = (int64_t)cta.bid() * S::FPC; base < p.total_frames;
          base += stride_frames, g += stride_frames, s += ds, f += df) {
@@ -230,7 +245,27 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
         const float* src = p.in + (active ? s * p.signal_stride + start : 0);
 
         float2 v[R];
-        if (bulk) {
+        if constexpr (HALF) {
+            const int valid = active ? half_valid(f) : 0;
+            const int staged = bulk ? valid & ~3 : 0;
+            if (staged > 0) {
+                if (!cta.bulk_wait(bar, phase) && p.error_flag != nullptr) *p.error_flag = 1;
+                phase ^= 1;
+            }
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                v[q] = make_float2(0.f, 0.f);
+                if (q < R / 2) {
+                    const int i0 = 2 * (t + q * T);
+                    if (i0 < staged) {
+                        v[q] = stage_slot[t + q * T];
+                    } else {
+                        if (i0 < valid) v[q].x = MA_LDG(src + i0);
+                        if (i0 + 1 < valid) v[q].y = MA_LDG(src + i0 + 1);
+                    }
+                }
+            }
+        } else if (bulk) {
             if (active) {
                 if (!cta.bulk_wait(bar, phase) && p.error_flag != nullptr) *p.error_flag = 1;
                 phase ^= 1;
@@ -271,8 +306,7 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
                         fn -= p.frames_per_signal;
                         ++sn;
                     }
-                    cta.bulk_copy(stage_slot, p.in + sn * p.signal_stride + fn * (int64_t)p.hop,
-                                  N * (uint32_t)sizeof(float), bar);
+                    start_copy(sn, fn);
                 }
             };
             fft_run<P, 1, false, true, Cta, TWALU>(v, t, sbuf0, S::BUF_STRIDE, parity, p.twM, cta, twb, issue_next);
@@ -833,21 +867,30 @@ MA_HD void istft_body(const C2RParams& p, Cta& cta, float2* smem) {
 //    global memory through L1 instead, to afford a second exchange buffer, measured 27 % slower:
 //    the loads' latency is exposed at four warps per scheduler.)
 //  * OVT == 0: ring [R][T] float2 in shared memory, window in registers.
-// smem: exchange buffer | ring or window table [R*T] float2 | staged row [M+2] float2 | mbarrier.
-template <int M, int OVT = 0>
+//  * PLAIN: no window and no normalisation (window == nullptr, floor < 0), the block overlap-add of
+//    partitioned convolution: register ring, neither a window table nor divisions, the freed shared
+//    memory is a second exchange buffer (one barrier per exchange), and rows may start on odd samples.
+// smem: exchange buffer(s) | ring or window table [R*T] float2 | staged row [M+2] float2 | mbarrier.
+template <int M, int OVT = 0, bool PLAIN = false>
 struct IstftFastShape {
     using P = FftPlan<M>;
     static constexpr bool REGRING = OVT > 0;
     static constexpr int ELEMS = smem_elems_per_fft<M, 1>();
-    static constexpr int RING = P::R * P::T;  // the ring, or (REGRING) the window table
+    static constexpr int RING = PLAIN ? 0 : P::R * P::T;  // the ring, or (REGRING) the window table
     static constexpr int ROW = M + 2;  // staged spectrum row with the alignment slack
-    static constexpr int EXCH = 1;  // exchange buffers (1: a barrier before each write instead of a second buffer)
+    static constexpr int EXCH = PLAIN ? 2 : 1;  // exchange buffers (1: a barrier before each write instead of a second buffer)
     static constexpr int EXCH_ELEMS = (EXCH * ELEMS + 1) & ~1;  // keeps the staged row 16-byte aligned
     static constexpr int TW1 = stage1_table_elems<FftPlanRev<M>>();  // stage-1 twiddle table behind the mbarrier
     static constexpr int SMEM_BYTES = (EXCH_ELEMS + RING + ROW + TW1) * (int)sizeof(float2) + 16;
     static_assert(!plan_pairable<M>() || ((EXCH_ELEMS + RING) * sizeof(float2)) % 16 == 0,
                   "bulk copy destination must be 16-byte aligned");
 };
+
+// Whether these parameters are the convolution's block overlap-add (PLAIN with an overlap count of 2).
+template <int M>
+inline bool istft_plain(const C2RParams& p) {
+    return plan_pairable<M>() && p.layout == LAYOUT_HALF_PACKED && p.window == nullptr && p.floor < 0.f && p.hop == M && p.n_partials <= 1;
+}
 
 // Whether istft_fast_body serves these parameters.
 template <int M>
@@ -864,6 +907,7 @@ inline bool istft_fast_ok(const C2RParams& p) {
         if (p.n_partials > 1 || p.hop <= 0 || p.hop % (2 * T) != 0) return false;
         const int h = p.hop / (2 * T);
         if (h > R || R % h != 0) return false;
+        if (istft_plain<M>(p)) return true;
         if ((reinterpret_cast<uintptr_t>(p.out) & 7) != 0 || (p.out_signal_stride & 1) != 0) return false;
         return true;
     }
@@ -876,10 +920,11 @@ MA_HD void store_pair_before(float* o, float2 r, int64_t left) {
     else if (left == 1) *o = r.x;
 }
 
-template <int M, int LAYOUT, int OVT, class Cta>
+template <int M, int LAYOUT, int OVT, class Cta, bool PLAIN = false>
 MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
     using P = FftPlan<M>;
-    using SH = IstftFastShape<M, OVT>;
+    using SH = IstftFastShape<M, OVT, PLAIN>;
+    static_assert(!PLAIN || OVT > 0, "the plain overlap-add keeps its ring in registers");
     constexpr int R = P::R, T = P::T, N = 2 * M;
     constexpr bool REGRING = SH::REGRING;
     // Every layout stages the next frame's spectrum row(s) with bulk copies: one copy of the complex
@@ -909,10 +954,12 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
     const int hop = p.hop;
     const int h = OVT > 0 ? R / OVT : hop / (2 * T);  // ring slots completed per frame
     const int64_t F = p.frames_per_signal;
-    const bool normalise = !(p.window == nullptr && p.floor < 0.f);
+    const bool normalise = !PLAIN && !(p.window == nullptr && p.floor < 0.f);
 
     float2 wreg[REGRING ? 1 : R];
-    if constexpr (REGRING) {
+    if constexpr (PLAIN) {
+        (void)wreg;
+    } else if constexpr (REGRING) {
         // window table into shared memory, once: entry [q2*T + t] is read by thread t alone
         float4* wtab = reinterpret_cast<float4*>(ring);
 #pragma unroll
@@ -998,7 +1045,8 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
                 p, true, s, f, G, t, smem, SH::ELEMS, parity, v, cta, twb, wherm, stage, issue_next, nullptr, tw1);
         } else {
             const StagedRow r = staged_row<M>(p, s, f);
-            c2r_frame<M, LAYOUT, true, Cta, true, decltype(issue_next), SH::EXCH == 1, true>(
+            // PLAIN: exact twiddles, as in the convolution's forward transform (see r2c_body)
+            c2r_frame<M, LAYOUT, !PLAIN, Cta, true, decltype(issue_next), SH::EXCH == 1, true>(
                 p, true, s, f, G, t, smem, SH::ELEMS, parity, v, cta, twb, wherm, stage + r.shift, issue_next, r.row, tw1);
         }
 
@@ -1010,6 +1058,28 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
         // every sample this frame completes has all its overlapping frames present
         const bool interior = !last && start >= (int64_t)(N - hop);
         float* out = p.out + s * p.out_signal_stride + start;
+        if constexpr (PLAIN) {
+            const float2 sc = make_float2(scale, scale);
+            const bool even = (reinterpret_cast<uintptr_t>(out) & 7) == 0;  // hop is even: the same for a whole row
+#pragma unroll
+            for (int q = 0; q < R; ++q) {
+                const float2 acc = q < R - HR ? pfma(v[q], sc, racc[q]) : pmul(v[q], sc);
+                const int i0 = 2 * (t + q * T);
+                if (emit && !last && q < HR) {
+                    if (even) {
+                        *reinterpret_cast<float2*>(out + i0) = make_float2(acc.y, acc.x);
+                    } else {
+                        out[i0] = acc.y;
+                        out[i0 + 1] = acc.x;
+                    }
+                } else if (emit && last) {
+                    if (start + i0 < p.out_len) out[i0] = acc.y;
+                    if (start + i0 + 1 < p.out_len) out[i0 + 1] = acc.x;
+                }
+                if (q >= HR) racc[q - HR] = acc;
+            }
+            continue;
+        }
         if constexpr (REGRING) {
             const float4* wtab = reinterpret_cast<const float4*>(ring) + t;
             if (emit && interior && normalise) {

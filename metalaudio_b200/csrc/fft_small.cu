@@ -53,11 +53,11 @@ static void launch_maybe_dependent(K kernel, int grid, int threads, size_t smem,
     (void)cudaLaunchKernelEx(&cfg, kernel, p);  // an error is picked up by after_launch
 }
 
-template <int M, bool ALIGNED, int LAYOUT, int MAGK>
+template <int M, bool ALIGNED, int LAYOUT, int MAGK, bool HALF>
 __global__ void __launch_bounds__(CtaShape<M>::THREADS, 512 / CtaShape<M>::THREADS) r2c_kernel(const R2CParams p) {
     DevCta cta;
     if (p.dependent_launch) dependents_launch();
-    r2c_body<M, ALIGNED, LAYOUT, MAGK, DevCta>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
+    r2c_body<M, ALIGNED, LAYOUT, MAGK, DevCta, HALF>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
     if (p.dependent_launch) dependency_wait();
 }
 
@@ -77,12 +77,12 @@ __global__ void __launch_bounds__(FftPlan<M>::T, (512 / FftPlan<M>::T) > 16 ? 16
     istft_body<M, DevCta>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
 }
 
-template <int M, int LAYOUT, int OVT>
+template <int M, int LAYOUT, int OVT, bool PLAIN = false>
 __global__ void __launch_bounds__(FftPlan<M>::T, (512 / FftPlan<M>::T) > 16 ? 16 : (512 / FftPlan<M>::T))
 istft_fast_kernel(const C2RParams p) {
     DevCta cta;
     if constexpr (plan_pairable<M>())
-        istft_fast_body<M, LAYOUT, OVT, DevCta>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
+        istft_fast_body<M, LAYOUT, OVT, DevCta, PLAIN>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
 }
 
 // Resident CTAs per SM for a kernel (cached per instantiation and device), after raising
@@ -96,19 +96,21 @@ static ma_status occupancy(K kernel, int threads, size_t smem, int* per_sm) {
     return MA_OK;
 }
 
-template <int M, bool ALIGNED, int LAYOUT, int MAGK>
-static ma_status launch_r2c_t(ma_fft_plan* plan, const R2CParams& p) {
+template <int M, bool ALIGNED, int LAYOUT, int MAGK, bool HALF = false>
+static ma_status launch_r2c_t(ma_fft_plan* plan, R2CParams p) {
     using S = CtaShape<M>;
     static int per_sm[64] = {0};
     ma_context* ctx = plan->ctx;
     int& occ = per_sm[ctx->device & 63];
     constexpr size_t smem = (ALIGNED && LAYOUT >= 0 && plan_pairable<M>()) ? S::SMEM_BYTES_PREFETCH : S::SMEM_BYTES;
-    if (occ == 0) MA_TRY(occupancy(r2c_kernel<M, ALIGNED, LAYOUT, MAGK>, S::THREADS, smem, &occ));
+    if (occ == 0) MA_TRY(occupancy(r2c_kernel<M, ALIGNED, LAYOUT, MAGK, HALF>, S::THREADS, smem, &occ));
     int64_t want = (p.total_frames + S::FPC - 1) / S::FPC;
     int64_t cap = (int64_t)ctx->sm_count * occ;
     int grid = (int)(want < cap ? want : cap);
     if (grid < 1) return MA_OK;
-    launch_maybe_dependent(r2c_kernel<M, ALIGNED, LAYOUT, MAGK>, grid, S::THREADS, smem, ctx->stream, p, p.dependent_launch);
+    // One frame per CTA: nothing to fetch ahead, the threads' own loads arrive sooner than a staged copy.
+    if (HALF && want <= cap) p.bulk_ok = 0;
+    launch_maybe_dependent(r2c_kernel<M, ALIGNED, LAYOUT, MAGK, HALF>, grid, S::THREADS, smem, ctx->stream, p, p.dependent_launch);
     return after_launch(ctx);
 }
 
@@ -127,6 +129,9 @@ static ma_status launch_r2c_variant(ma_fft_plan* plan, const R2CParams& p, bool 
             MA_R2C_CASE(LAYOUT_HALF_POLAR, -1)
 #undef MA_R2C_CASE
         }
+        // the convolution's zero-padded blocks
+        if (!aligned && magk == -1 && p.layout == LAYOUT_HALF_PACKED && p.frame_valid == M && p.window == nullptr)
+            return launch_r2c_t<M, true, LAYOUT_HALF_PACKED, -1, true>(plan, p);
     }
     return aligned ? launch_r2c_t<M, true, -1, -2>(plan, p) : launch_r2c_t<M, false, -1, -2>(plan, p);
 }
@@ -139,7 +144,7 @@ ma_status launch_r2c_small(ma_fft_plan* plan, R2CParams p) {
     const int64_t last_end = (p.frames_per_signal - 1) * (int64_t)p.hop + n;
     const bool aligned = ((uintptr_t)p.in % 8 == 0) && (p.signal_stride % 2 == 0) && (p.hop % 2 == 0) &&
                          p.frame_valid >= n && last_end <= p.signal_len;
-    p.bulk_ok = (aligned && (uintptr_t)p.in % 16 == 0 && p.signal_stride % 4 == 0 && p.hop % 4 == 0 && n % 4 == 0) ? 1 : 0;
+    p.bulk_ok = ((aligned || p.frame_valid == n / 2) && (uintptr_t)p.in % 16 == 0 && p.signal_stride % 4 == 0 && p.hop % 4 == 0 && n % 4 == 0) ? 1 : 0;
     p.error_flag = plan->ctx->d_error_flag;
     ma_status st = MA_ERR_UNSUPPORTED;
     // Aligned launches of the paired plans get kernels with the layout and the magnitude kind
@@ -201,20 +206,23 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     const bool fast = istft_fast_ok<M>(p);
     const int ov = fast ? (2 * M) / p.hop : 0;
     // 0: general kernel; 1: fast, overlap count read at run time; 2: fast with the overlap count 4
-    // fixed at compile time (register ring)
-    const int kind = !fast ? 0 : (ov == 4 ? 2 : 1);
-    const size_t smem = kind == 2 ? (size_t)IstftFastShape<M, 4>::SMEM_BYTES
+    // fixed at compile time (register ring); 3: the convolution's block overlap-add
+    const int kind = !fast ? 0 : istft_plain<M>(p) ? 3 : (ov == 4 ? 2 : 1);
+    const size_t smem = kind == 3 ? (size_t)IstftFastShape<M, 2, true>::SMEM_BYTES
+                      : kind == 2 ? (size_t)IstftFastShape<M, 4>::SMEM_BYTES
                       : kind == 1 ? (size_t)IstftFastShape<M, 0>::SMEM_BYTES
                                   : 2 * smem_elems_per_fft<M, 1>() * sizeof(float2) + 2 * M * sizeof(float);
-    static int per_sm[3][64] = {{0}, {0}, {0}};
+    static int per_sm[4][64] = {{0}, {0}, {0}, {0}};
     ma_context* ctx = plan->ctx;
     int& occ = per_sm[kind][ctx->device & 63];
-    const int variant = !fast ? 0
+    const int variant = !fast || kind == 3 ? 0
                               : (p.layout == LAYOUT_HALF_INTERLEAVED ? 1 : (p.layout == LAYOUT_HALF_PACKED ? 3 : 5)) +
                                     (ov == 4 ? 1 : 0);
     if (occ == 0) {  // the layout variants of a kind share its footprint; raise every one's shared-memory limit
         int dummy;
-        if (kind == 2) {
+        if (kind == 3) {
+            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true>, T, smem, &occ));
+        } else if (kind == 2) {
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 4>, T, smem, &occ));
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 4>, T, smem, &dummy));
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_POLAR, 4>, T, smem, &dummy));
@@ -243,6 +251,10 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     }
     int grid = (int)(total < cap ? total : cap);
     if (grid < 1) return MA_OK;
+    if (kind == 3) {
+        istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true><<<grid, T, smem, ctx->stream>>>(p);
+        return after_launch(ctx);
+    }
     switch (variant) {
         case 1: istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0><<<grid, T, smem, ctx->stream>>>(p); break;
         case 2: istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 4><<<grid, T, smem, ctx->stream>>>(p); break;

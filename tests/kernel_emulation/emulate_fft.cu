@@ -2,6 +2,7 @@
 // TEST INFRASTRUCTURE ONLY (built by tests/test_kernel_emulation.py into a private .so).
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "../../metalaudio_b200/csrc/fft_kernels.cuh"
@@ -112,6 +113,42 @@ int emul_istft(int n, int hop, const float* in_a, const float* in_b, long long i
     MA_DISPATCH_M(M, RUN)
 #undef RUN
     return rc == 0 ? used_fast : rc;
+}
+
+// The convolution's transforms of the paired plans: zero-padded blocks -> packed spectra (`spec`, [signals][blocks][M])
+// and their plain block overlap-add, cut at out_len.  -1 for lengths without a paired plan.
+int emul_conv_blocks(int n, const float* in, long long signal_stride, long long signal_len, long long blocks, long long n_signals,
+                     int bulk_ok, float* spec, float* out, long long out_signal_stride, long long out_len, int nblocks) {
+    const int M = n / 2;
+    auto twM = make_stage_tables_for(M, false), twI = make_stage_tables_for(M, true);
+    auto twN = make_hermitian_table(M);
+    R2CParams p{};
+    p.in = in; p.signal_stride = signal_stride; p.frames_per_signal = blocks; p.total_frames = blocks * n_signals;
+    p.signal_len = signal_len; p.hop = M; p.frame_valid = M; p.out_a = spec; p.out_signal_stride = blocks * M; p.out_frame_stride = M;
+    p.layout = LAYOUT_HALF_PACKED; p.mag_kind = MAG_NONE; p.bulk_ok = bulk_ok; p.twM = twM.data(); p.twN = twN.data();
+    C2RParams c{};
+    c.in_a = spec; c.in_signal_stride = blocks * M; c.in_frame_stride = M; c.frames_per_signal = blocks; c.n_signals = n_signals;
+    c.layout = LAYOUT_HALF_PACKED; c.hop = M; c.out = out; c.out_signal_stride = out_signal_stride; c.out_len = out_len;
+    c.floor = -1.f; c.twM = twI.data(); c.twN = twN.data();
+    int rc = -1;
+    auto run = [&](auto length) {
+        constexpr int MM = decltype(length)::value;
+        if constexpr (plan_pairable<MM>()) {
+            using S = CtaShape<MM>;
+            if (!istft_plain<MM>(c) || !istft_fast_ok<MM>(c)) return;
+            run_grid(nblocks, S::THREADS, S::SMEM_BYTES_PREFETCH, [&](HostCta& cta, void* sm) {
+                r2c_body<MM, true, LAYOUT_HALF_PACKED, -1, HostCta, true>(p, cta, (float2*)sm);
+            });
+            run_grid(nblocks, S::T, IstftFastShape<MM, 2, true>::SMEM_BYTES, [&](HostCta& cta, void* sm) {
+                istft_fast_body<MM, LAYOUT_HALF_PACKED, 2, HostCta, true>(c, cta, (float2*)sm);
+            });
+            rc = 0;
+        }
+    };
+#define RUN(MM) run(std::integral_constant<int, MM>{});
+    MA_DISPATCH_M(M, RUN)
+#undef RUN
+    return rc;
 }
 
 // Walks the staging schedule of the time-tiled multiply-accumulate for P partitions and t_total

@@ -41,6 +41,7 @@ def emul():
     lib.emul_c2r.argtypes = [ctypes.c_int, FP, FP, LL, LL, LL, LL, ctypes.c_int, FP, ctypes.c_int]
     lib.emul_istft.argtypes = [ctypes.c_int, ctypes.c_int, FP, FP, LL, LL, LL, LL, ctypes.c_int, FP, ctypes.c_float,
                                FP, LL, LL, ctypes.c_int, ctypes.c_int]
+    lib.emul_conv_blocks.argtypes = [ctypes.c_int, FP, LL, LL, LL, LL, ctypes.c_int, FP, FP, LL, LL, ctypes.c_int]
     lib.emul_tiled_rows.argtypes = [ctypes.c_int, LL, ctypes.POINTER(LL)]
     lib.emul_tiled_rows.restype = LL
     return lib
@@ -115,6 +116,33 @@ def test_stft_istft(emul, n, hop, length, chunks, kind):
     ws = rp.window_sum(f, n, hop, w, 0.0)
     msk = ws >= 1e-2 * ws.max()
     assert o64.rel_rms(y[:, msk], yref[:, msk]) <= 1e-5
+
+
+@pytest.mark.parametrize("n", [64, 256, 1024, 2048, 4096])
+@pytest.mark.parametrize("length_off,stride_mod,cut", [(0, 0, 0), (-1, 0, 1), (3, 1, 2), (-5, 3, 7)])
+def test_convolution_block_transforms(emul, n, length_off, stride_mod, cut):
+    """Zero-padded blocks in, plain block overlap-add out, on the paired plans: rows on and off the
+    16-byte grid, a ragged last block, blocks wholly behind the input, rows that end on odd samples."""
+    b = n // 2
+    signals, blocks = 3, 6
+    length = 4 * b + length_off
+    stride = (length + 7) // 4 * 4 + stride_mod
+    rng = np.random.default_rng(n + length)
+    x = rng.standard_normal((signals, stride)).astype(np.float32)
+    spec = np.zeros((signals, blocks, b, 2), np.float32)
+    out_len = blocks * b - cut
+    y = np.full((signals, out_len), 7.0, np.float32)
+    for bulk in ([0, 1] if stride_mod == 0 else [0]):
+        spec[:] = 0
+        y[:] = 7.0
+        assert emul.emul_conv_blocks(n, fp(x), stride, length, blocks, signals, bulk, fp(spec), fp(y), out_len, out_len, 4) == 0
+        padded = np.zeros((signals, blocks, n))
+        tail = np.zeros((signals, blocks * b)); tail[:, :length] = x[:, :length]
+        padded[..., :b] = tail.reshape(signals, blocks, b)
+        ref = np.fft.rfft(padded, axis=-1)
+        assert o64.rel_rms(spec[..., 1:, 0] + 1j * spec[..., 1:, 1], ref[..., 1:b]) <= 1e-6
+        assert np.allclose(spec[..., 0, 1], ref[..., b].real, atol=1e-3)
+        assert o64.rel_rms(y, tail[:, :out_len]) <= 1e-6
 
 
 @pytest.mark.parametrize("n,cut", [(256, 1), (256, 130), (256, 200), (1024, 777), (4096, 4000)])
