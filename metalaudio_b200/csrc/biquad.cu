@@ -43,6 +43,10 @@ constexpr int kBqMaxSections = 32;
 //   [8..135]   A^(PER*l) row-major 2x2, l < 32 (PER: samples per thread)
 //   [136..139] A^(PER*32)
 //   [140..171] A^(PER*32*w), w < 8: a warp's worth of samples, w times over
+// Time splits (few channels): cascades of up to kBqSplitSections sections; a ladder of kBqLadder matrices per
+// coefficient set, entry j the zero-input transition of the whole cascade (2S x 2S, row-major, state
+// order z1 z2 of section 0, z1 z2 of section 1, ...) over 2^j tiles.
+constexpr int kBqSplitSections = 8, kBqLadder = 9, kBqMaxChunks = 64;
 constexpr int kBqCoef = 0, kBqPl = 8, kBqPw = 136, kBqPx = 140, kBqTable = 172;
 
 struct BiquadLaunch {
@@ -53,7 +57,15 @@ struct BiquadLaunch {
     const int32_t* channel_to_set;
     float2* state;                // [n_channels][n_sections]
     int32_t n_sections;
+    // time splits
+    int32_t chunks, chunk_tiles;  // chunks per channel; tiles per chunk (the last one may be shorter)
+    const double* ladder;         // [n_sets][kBqLadder][2S][2S]
+    double2* ends;                // [n_channels][chunks][n_sections]: [0] the state in front of the call, [k + 1] the
+                                  // state chunk k reaches from zero
 };
+
+// Which part of a channel a CTA filters.
+enum { BQ_WHOLE = 0, BQ_ENDS = 1, BQ_CHUNK = 2 };
 
 __device__ __forceinline__ double2 mat_vec(const double* m, double2 v) {
     return make_double2(fma(m[0], v.x, m[1] * v.y), fma(m[2], v.x, m[3] * v.y));
@@ -68,6 +80,59 @@ __device__ __forceinline__ int swizzled(int i) {
     return (((r << 3) | ((g & 7) ^ (r & 7))) << 2) | (i & 3);
 }
 
+// The state in front of chunk `chunk` of a channel: s_0 = ends[0], s_{k+1} = M s_k + ends[k + 1], M the product
+// of the ladder matrices that make up one chunk.  `scratch` takes 2 * 16 * 16 + kBqMaxChunks * 16 doubles (12 KB).
+// Called by the whole CTA; the results are visible after the caller's next barrier.
+__device__ __forceinline__ void chunk_start_state(const BiquadLaunch& p, int set, int chunk, const double2* ends,
+                                                  double* scratch, double2* carry) {
+    constexpr int kMax = 2 * kBqSplitSections;
+    static_assert(kMax * kMax == kBqThreads, "one thread per matrix entry");
+    const int tid = threadIdx.x, S = p.n_sections, D = 2 * S;
+    const int r = tid / kMax, c = tid % kMax;
+    const bool entry = r < D && c < D;
+    double* e = scratch + 2 * kMax * kMax;
+    const double* ge = reinterpret_cast<const double*>(ends);
+    for (int i = tid; i < (chunk + 1) * D; i += kBqThreads) e[i] = ge[i];
+    const double* ladder = p.ladder + (int64_t)set * kBqLadder * D * D;
+    double m = 0.0;
+    int cur = 0;
+    bool first = true;
+    for (int j = 0; j < kBqLadder; ++j) {
+        if (!((p.chunk_tiles >> j) & 1)) continue;
+        const double* L = ladder + j * D * D;
+        if (entry) {
+            if (first) {
+                m = __ldg(L + r * D + c);
+            } else {
+                m = 0.0;
+                for (int k = 0; k < D; ++k) m = fma(__ldg(L + r * D + k), scratch[cur * kMax * kMax + k * kMax + c], m);
+            }
+            scratch[(cur ^ 1) * kMax * kMax + r * kMax + c] = m;
+        }
+        first = false;
+        cur ^= 1;
+        __syncthreads();
+    }
+    if (tid < 32) {
+        double row[kMax];
+#pragma unroll
+        for (int k = 0; k < kMax; ++k) row[k] = tid < D && k < D ? scratch[cur * kMax * kMax + tid * kMax + k] : 0.0;
+        double v = tid < D ? e[tid] : 0.0;
+        for (int j = 1; j <= chunk; ++j) {
+            double a0 = tid < D ? e[j * D + tid] : 0.0, a1 = 0.0;
+#pragma unroll
+            for (int k = 0; k < kMax; k += 2) {
+                if (k < D) {
+                    a0 = fma(row[k], __shfl_sync(0xffffffffu, v, k), a0);
+                    a1 = fma(row[k + 1], __shfl_sync(0xffffffffu, v, k + 1), a1);
+                }
+            }
+            v = a0 + a1;
+        }
+        if (tid < D) reinterpret_cast<double*>(carry)[tid] = v;
+    }
+}
+
 // Why double precision inside: a thread restarts the recurrence every 32 samples.  In float32 the
 // rounding drift of one block and the freshly computed state of the next do not line up, which
 // leaves a small step at every block boundary; a later section that rejects the band the signal
@@ -75,7 +140,15 @@ __device__ __forceinline__ int swizzled(int i) {
 // order of magnitude further from the exact filter than the serial float32 walk.  With the state
 // in double the steps vanish and every section's output is the exact filter's, rounded once to
 // float32 (the precision sections exchange data in, as the reference's float arrays do).
-template <int kBqPer, bool DBL>
+//
+// One CTA per channel leaves most of the device idle below about 150 channels, and a channel is a long
+// serial chain of tiles.  There the time axis is cut into chunks of whole tiles as well (MODE):
+//   BQ_ENDS   filters every chunk but the last from a zero state and keeps only the end state of the cascade
+//             (no output; the last section stops at its end state);
+//   BQ_CHUNK  one warp walks s_{k+1} = M s_k + e_k over the chunks in front, M the cascade's transition over
+//             one chunk, and the chunk is then filtered as usual from that state.
+// The arithmetic doubles but runs on every SM, so three chunks and more are faster than one CTA.
+template <int kBqPer, bool DBL, int MODE>
 __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunch p) {
     constexpr int kBqTile = kBqThreads * kBqPer;
     using X = typename std::conditional<DBL, double, float>::type;  // how a thread holds its samples between sections
@@ -85,16 +158,29 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
     double2* carry = warp_end + 2 * kBqWarps;                           // [2][n_sections]: read one, write the other
     float* tiles = reinterpret_cast<float*>(carry + 2 * p.n_sections);  // two tiles: one in use, one being filled
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t ch = blockIdx.x;
+    const int64_t ch = MODE == BQ_WHOLE ? blockIdx.x : blockIdx.y;
+    const int chunk = MODE == BQ_WHOLE ? 0 : (int)blockIdx.x;
     const int set = p.channel_to_set != nullptr ? p.channel_to_set[ch] : 0;
     const double* gtab = p.tables + (int64_t)set * p.n_sections * kBqTable;
     for (int i = tid; i < p.n_sections * kBqTable; i += kBqThreads) tab[i] = __ldg(gtab + i);
-    for (int s = tid; s < p.n_sections; s += kBqThreads) {
-        const float2 z = p.state[ch * p.n_sections + s];
-        carry[s] = make_double2((double)z.x, (double)z.y);
+    double2* ends = p.ends + ch * p.chunks * p.n_sections;
+    if constexpr (MODE == BQ_CHUNK) {
+        chunk_start_state(p, set, chunk, ends, reinterpret_cast<double*>(tiles + kBqTile), carry);
+    } else {
+        for (int s = tid; s < p.n_sections; s += kBqThreads) {
+            const float2 z = p.state[ch * p.n_sections + s];
+            const double2 zd = make_double2((double)z.x, (double)z.y);
+            carry[s] = MODE == BQ_ENDS ? make_double2(0.0, 0.0) : zd;
+            if (MODE == BQ_ENDS && chunk == 0) ends[s] = zd;  // the last chunk's CTA overwrites p.state later
+        }
     }
-    const float* in = p.in + ch * p.in_stride;
-    float* out = p.out + ch * p.out_stride;
+    const int64_t skipped = (int64_t)chunk * p.chunk_tiles * kBqTile;
+    const int64_t samples = MODE == BQ_WHOLE ? p.samples
+                          : p.samples - skipped < (int64_t)p.chunk_tiles * kBqTile ? p.samples - skipped
+                                                                                   : (int64_t)p.chunk_tiles * kBqTile;
+    const bool ends_signal = MODE == BQ_WHOLE || (MODE == BQ_CHUNK && chunk == p.chunks - 1);
+    const float* in = p.in + ch * p.in_stride + skipped;
+    float* out = p.out + ch * p.out_stride + skipped;
     const bool vec_in = (reinterpret_cast<uintptr_t>(in) & 15) == 0;
     const bool vec_out = (reinterpret_cast<uintptr_t>(out) & 15) == 0;
     __syncthreads();
@@ -111,18 +197,18 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
         }
         __pipeline_commit();
     };
-    auto full_tile = [&](int64_t base) { return vec_in && base + kBqTile <= p.samples; };
+    auto full_tile = [&](int64_t base) { return vec_in && base + kBqTile <= samples; };
     bool fetched = false;
-    if (p.samples > 0 && full_tile(0)) {
+    if (samples > 0 && full_tile(0)) {
         prefetch(0, tiles);
         fetched = true;
     }
     int par = 0;
-    for (int64_t base = 0; base < p.samples; base += kBqTile, par ^= 1) {
+    for (int64_t base = 0; base < samples; base += kBqTile, par ^= 1) {
         float* tile = tiles + par * kTileFloats;
         const double2* carry_in = carry + par * p.n_sections;
         double2* carry_out = carry + (par ^ 1) * p.n_sections;
-        const int64_t left = p.samples - base;
+        const int64_t left = samples - base;
         const int valid = left < kBqTile ? (int)left : kBqTile;
         // ---- this tile: already on its way, or loaded here (ragged / unaligned: zeros beyond the end)
         if (fetched) {
@@ -136,7 +222,7 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
         }
         // ---- next tile: start it now (its buffer was last read two iterations ago, before the barriers since)
         fetched = false;
-        if (base + kBqTile < p.samples && full_tile(base + kBqTile)) {
+        if (base + kBqTile < samples && full_tile(base + kBqTile)) {
             prefetch(base + kBqTile, tiles + (par ^ 1) * kTileFloats);
             fetched = true;
         }
@@ -216,6 +302,16 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
                     c = make_double2(m.x + wend[w].x, m.y + wend[w].y);
                 }
             }
+            if (MODE == BQ_ENDS && s == p.n_sections - 1) {
+                // nobody reads this section's output: its state at the end of the tile is enough
+                if (tid == kBqThreads - 1) {
+                    const double2 m = mat_vec(T + kBqPw, c);
+                    const double2 z = make_double2(e.x + m.x, e.y + m.y);
+                    if (last_tile) ends[(int64_t)(chunk + 1) * p.n_sections + s] = z;
+                    else carry_out[s] = z;
+                }
+                continue;
+            }
             double2 prev = make_double2(__shfl_up_sync(0xffffffffu, e.x, 1), __shfl_up_sync(0xffffffffu, e.y, 1));
             if (lane == 0) prev = make_double2(0.0, 0.0);
             const double2 pc = mat_vec(T + kBqPl + 4 * lane, c);
@@ -240,9 +336,11 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
                     }
                 }
             };
-            if (last_tile) second_pass(std::true_type{});
+            if (ends_signal && last_tile) second_pass(std::true_type{});
             else second_pass(std::false_type{});
-            if (owns_last) {
+            if (MODE == BQ_ENDS && last_tile && tid == kBqThreads - 1)  // chunks that are not the last are whole tiles
+                ends[(int64_t)(chunk + 1) * p.n_sections + s] = make_double2(s1, s2);
+            if (ends_signal && owns_last) {
                 // results below the smallest normal are stored as zero (DSP.metal:736-740)
                 float g1 = (float)f1, g2 = (float)f2;
                 if (fabsf(g1) < 1.17549435e-38f) g1 = 0.f;
@@ -251,6 +349,10 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
             }
             // carry for the next tile: the state the last thread ends in
             if (!last_tile && tid == kBqThreads - 1) carry_out[s] = make_double2(s1, s2);
+        }
+        if constexpr (MODE == BQ_ENDS) {
+            __syncthreads();  // the tile and the carries are reused by the next iteration
+            continue;
         }
         // ---- contiguous store through the same tile
 #pragma unroll
@@ -315,6 +417,47 @@ static void build_table(const float* c, double* t, int per) {
     }
 }
 
+// Zero-input transition of a cascade over 2^j tiles, j < kBqLadder (see kBqLadder).  False when a section is
+// not strictly stable: its powers need not stay finite over thousands of samples.
+static bool build_ladder(const float* coeffs, int sections, int tile, double* ladder) {
+    const int D = 2 * sections;
+    std::vector<double> a((size_t)D * D, 0.0), b((size_t)D * D);
+    // column i of the one-sample transition: the cascade's next state from unit state i and no input
+    for (int i = 0; i < D; ++i) {
+        double x = 0.0;
+        for (int s = 0; s < sections; ++s) {
+            const float* c = coeffs + 5 * s;
+            const double z1 = i == 2 * s ? 1.0 : 0.0, z2 = i == 2 * s + 1 ? 1.0 : 0.0;
+            const double y = (double)c[0] * x + z1;
+            a[(size_t)(2 * s) * D + i] = (double)c[1] * x - (double)c[3] * y + z2;
+            a[(size_t)(2 * s + 1) * D + i] = (double)c[2] * x - (double)c[4] * y;
+            x = y;
+        }
+    }
+    for (int s = 0; s < sections; ++s) {
+        const double a1 = coeffs[5 * s + 3], a2 = coeffs[5 * s + 4];
+        if (!(std::fabs(a2) < 1.0 && std::fabs(a1) < 1.0 + a2)) return false;
+    }
+    auto square = [&]() {
+        for (int r = 0; r < D; ++r)
+            for (int c = 0; c < D; ++c) {
+                double v = 0.0;
+                for (int k = 0; k < D; ++k) v += a[(size_t)r * D + k] * a[(size_t)k * D + c];
+                b[(size_t)r * D + c] = v;
+            }
+        a.swap(b);
+    };
+    for (int n = 1; n < tile; n *= 2) square();
+    for (int j = 0; j < kBqLadder; ++j) {
+        if (j > 0) square();
+        for (size_t i = 0; i < a.size(); ++i) {
+            if (!std::isfinite(a[i])) return false;
+            ladder[(size_t)j * D * D + i] = a[i];
+        }
+    }
+    return true;
+}
+
 }  // namespace ma
 
 using namespace ma;
@@ -326,12 +469,44 @@ struct ma_biquad {
     int32_t* d_map = nullptr;
     float2* d_state = nullptr;
     bool smem_raised = false;
+    double* d_ladder = nullptr;  // transitions for time splits; nullptr: the cascade is not split
+    double2* d_ends = nullptr;   // [2 * SMs][sections], the chunks' end states
     int per = kBqPerShort;  // samples per thread: the kernel variant, fixed by the section count
 };
 
 static size_t biquad_smem(int sections, int per) {
     return sizeof(float) * (size_t)(2 * kBqThreads * per) + sizeof(double) * (size_t)(sections * kBqTable) +
            sizeof(double2) * (size_t)(2 * kBqWarps + 2 * sections);
+}
+
+// Chunks per channel that fill the device once: two CTAs of 256 threads share an SM.
+constexpr int kBqSplitFrom = 3;
+static int split_max_chunks(const ma_biquad* bq) {
+    if (bq->sections > kBqSplitSections) return 1;
+    const int n = 2 * bq->ctx->sm_count / bq->channels;
+    return n < kBqMaxChunks ? n : kBqMaxChunks;
+}
+
+template <int PER, bool DBL>
+static ma_status launch_biquad(ma_biquad* bq, BiquadLaunch& p, size_t smem) {
+    cudaStream_t stream = bq->ctx->stream;
+    if (p.chunks > 1) {
+        biquad_kernel<PER, DBL, BQ_ENDS><<<dim3((unsigned)(p.chunks - 1), (unsigned)bq->channels), kBqThreads, smem, stream>>>(p);
+        MA_TRY(after_launch(bq->ctx));
+        biquad_kernel<PER, DBL, BQ_CHUNK><<<dim3((unsigned)p.chunks, (unsigned)bq->channels), kBqThreads, smem, stream>>>(p);
+    } else {
+        biquad_kernel<PER, DBL, BQ_WHOLE><<<(unsigned)bq->channels, kBqThreads, smem, stream>>>(p);
+    }
+    return after_launch(bq->ctx);
+}
+
+template <int PER, bool DBL>
+static ma_status raise_smem() {
+    const int bytes = (int)biquad_smem(kBqMaxSections, PER);
+    MA_CUDA(cudaFuncSetAttribute(biquad_kernel<PER, DBL, BQ_WHOLE>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MA_CUDA(cudaFuncSetAttribute(biquad_kernel<PER, DBL, BQ_ENDS>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    MA_CUDA(cudaFuncSetAttribute(biquad_kernel<PER, DBL, BQ_CHUNK>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    return MA_OK;
 }
 
 extern "C" {
@@ -349,6 +524,8 @@ ma_status ma_biquad_create(ma_context* ctx, int32_t n_channels, int32_t n_sectio
     bq->per = n_sections >= kBqLongFrom ? kBqPerLong : kBqPerShort;
     cudaError_t e = cudaMalloc((void**)&bq->d_state, sizeof(float2) * (size_t)n_channels * n_sections);
     if (e == cudaSuccess) e = cudaMemsetAsync(bq->d_state, 0, sizeof(float2) * (size_t)n_channels * n_sections, ctx->stream);  // ordered before the first kernel of the context
+    if (e == cudaSuccess && split_max_chunks(bq) >= kBqSplitFrom)
+        e = cudaMalloc((void**)&bq->d_ends, sizeof(double2) * (size_t)(2 * ctx->sm_count) * n_sections);
     if (e != cudaSuccess) {
         ma_biquad_destroy(bq);
         return cuda_fail(e);
@@ -362,6 +539,8 @@ ma_status ma_biquad_destroy(ma_biquad* bq) {
     if (bq->d_tables) (void)cudaFree(bq->d_tables);
     if (bq->d_map) (void)cudaFree(bq->d_map);
     if (bq->d_state) (void)cudaFree(bq->d_state);
+    if (bq->d_ladder) (void)cudaFree(bq->d_ladder);
+    if (bq->d_ends) (void)cudaFree(bq->d_ends);
     delete bq;
     return MA_OK;
 }
@@ -378,13 +557,28 @@ ma_status ma_biquad_set_coefficients(ma_biquad* bq, const float* coeffs, int32_t
             if (channel_to_set[c] < 0 || channel_to_set[c] >= n_sets) return MA_ERR_INVALID_ARGUMENT;
     std::vector<double> tables((size_t)n_sets * bq->sections * kBqTable);
     for (int64_t i = 0; i < (int64_t)n_sets * bq->sections; ++i) build_table(coeffs + 5 * i, tables.data() + kBqTable * i, bq->per);
+    std::vector<double> ladder;
+    if (split_max_chunks(bq) >= kBqSplitFrom) {
+        const size_t per_set = (size_t)kBqLadder * 4 * bq->sections * bq->sections;
+        ladder.resize(per_set * n_sets);
+        bool ok = true;
+        for (int64_t i = 0; i < n_sets && ok; ++i)
+            ok = build_ladder(coeffs + 5 * i * bq->sections, bq->sections, kBqThreads * bq->per, ladder.data() + per_set * i);
+        if (!ok) ladder.clear();
+    }
     MA_TRY(ma_context_sync(ctx, 30.0));  // nothing in flight may still read the old tables
     if (bq->d_tables) (void)cudaFree(bq->d_tables);
     if (bq->d_map) (void)cudaFree(bq->d_map);
+    if (bq->d_ladder) (void)cudaFree(bq->d_ladder);
     bq->d_tables = nullptr;
     bq->d_map = nullptr;
+    bq->d_ladder = nullptr;
     MA_CUDA(cudaMalloc((void**)&bq->d_tables, tables.size() * sizeof(double)));
     MA_TRY(copy_h2d(ctx, bq->d_tables, tables.data(), tables.size() * sizeof(double)));
+    if (!ladder.empty()) {
+        MA_CUDA(cudaMalloc((void**)&bq->d_ladder, ladder.size() * sizeof(double)));
+        MA_TRY(copy_h2d(ctx, bq->d_ladder, ladder.data(), ladder.size() * sizeof(double)));
+    }
     if (channel_to_set != nullptr) {
         MA_CUDA(cudaMalloc((void**)&bq->d_map, sizeof(int32_t) * (size_t)bq->channels));
         MA_TRY(copy_h2d(ctx, bq->d_map, channel_to_set, sizeof(int32_t) * (size_t)bq->channels));
@@ -406,12 +600,7 @@ ma_status ma_biquad_process_dev(ma_biquad* bq, const float* in, int64_t in_strid
     const size_t smem = biquad_smem(bq->sections, bq->per);
     const bool long_cascade = bq->per == kBqPerLong;
     if (!bq->smem_raised) {
-        if (long_cascade)
-            MA_CUDA(cudaFuncSetAttribute(biquad_kernel<kBqPerLong, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)biquad_smem(kBqMaxSections, kBqPerLong)));
-        else
-            MA_CUDA(cudaFuncSetAttribute(biquad_kernel<kBqPerShort, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)biquad_smem(kBqMaxSections, kBqPerShort)));
+        MA_TRY((long_cascade ? raise_smem<kBqPerLong, true>() : raise_smem<kBqPerShort, false>()));
         bq->smem_raised = true;
     }
     BiquadLaunch p{};
@@ -424,9 +613,24 @@ ma_status ma_biquad_process_dev(ma_biquad* bq, const float* in, int64_t in_strid
     p.channel_to_set = bq->d_map;
     p.state = bq->d_state;
     p.n_sections = bq->sections;
-    if (long_cascade) biquad_kernel<kBqPerLong, true><<<(unsigned)bq->channels, kBqThreads, smem, ctx->stream>>>(p);
-    else biquad_kernel<kBqPerShort, false><<<(unsigned)bq->channels, kBqThreads, smem, ctx->stream>>>(p);
-    return after_launch(ctx);
+    p.chunks = 1;
+    if (bq->d_ladder != nullptr) {
+        // Chunks write their part of a row while others still read theirs: the rows must be the same or apart.
+        const int64_t in_span = (bq->channels - 1) * in_stride + samples, out_span = (bq->channels - 1) * out_stride + samples;
+        const bool apart = in + in_span <= out || out + out_span <= in;
+        const bool same = in == out && (in_stride == out_stride || bq->channels == 1);
+        const int64_t tiles = (samples + kBqThreads * bq->per - 1) / (kBqThreads * bq->per);
+        const int64_t most = split_max_chunks(bq);
+        const int64_t per_chunk = (tiles + most - 1) / most;
+        const int64_t chunks = (tiles + per_chunk - 1) / per_chunk;
+        if ((apart || same) && chunks >= kBqSplitFrom && per_chunk < (1 << kBqLadder)) {
+            p.chunks = (int32_t)chunks;
+            p.chunk_tiles = (int32_t)per_chunk;
+            p.ladder = bq->d_ladder;
+            p.ends = bq->d_ends;
+        }
+    }
+    return long_cascade ? launch_biquad<kBqPerLong, true>(bq, p, smem) : launch_biquad<kBqPerShort, false>(bq, p, smem);
 }
 
 ma_status ma_biquad_process_host(ma_biquad* bq, const float* in, int64_t in_stride, float* out, int64_t out_stride,

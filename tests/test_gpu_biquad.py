@@ -179,3 +179,48 @@ def test_filter_bank_state_carries_between_series_and_parallel(device):
         FilterBank(device, bandCount=33)
     assert e.value.name == "bandCount"
     bank.close()
+
+
+@pytest.mark.parametrize("channels,sections", [(1, 1), (3, 2), (24, 4), (98, 3), (2, 8), (5, 9)])
+@pytest.mark.parametrize("tiles,extra", [(3, 0), (4, 1), (5, -1), (70, 5)])
+def test_time_splits_match_float64(device, lib, channels, sections, tiles, extra):
+    """Few channels: the time axis is cut into chunks that run on CTAs of their own (up to eight sections).
+    Edges of tiles and chunks, several coefficient sets, the state in front of and behind the call, in
+    place and into other rows.  A tile is 8192 samples, 4096 from three sections up."""
+    from metalaudio_b200 import Tensor
+    length = tiles * (4096 if sections >= 3 else 8192) + extra
+    if channels > 30 and tiles > 10:
+        channels = 30
+    rng = np.random.default_rng(100 * channels + sections + tiles)
+    kinds = [("lowpass", 0.0), ("peaking", 6.0), ("highpass", 0.0), ("lowshelf", -9.0)]
+    sets = min(channels, 3)
+    coef = np.stack([[rp.biquad_coefficients(kinds[(k + s) % 4][0], 60.0 * 2.0 ** ((k + s) % 8), 48000.0, 0.9, kinds[(k + s) % 4][1])
+                      for s in range(sections)] for k in range(sets)]).astype(np.float32)
+    of_channel = (np.arange(channels) % sets).astype(np.int32)
+    x = rng.standard_normal((channels, length)).astype(np.float32)
+    z0 = (0.01 * rng.standard_normal((channels, sections, 2))).astype(np.float32)
+    h = ctypes.c_void_p()
+    vp = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    assert lib.ma_biquad_create(device.handle, channels, sections, ctypes.byref(h)) == 0
+    try:
+        assert lib.ma_biquad_set_coefficients(h, vp(coef), sets, vp(of_channel)) == 0
+        ref = np.empty((channels, length))
+        zref = np.empty((channels, sections, 2))
+        for c in range(channels):
+            y = x[c].astype(np.float64)
+            for s in range(sections):
+                y, zref[c, s] = rp.biquad_process(y, coef[of_channel[c], s], z0[c, s].astype(np.float64), dtype=np.float64)
+            ref[c] = y
+        tin = Tensor(device, x.shape)
+        for in_place in (False, True):
+            tin.copy(x)
+            tout = tin if in_place else Tensor(device, x.shape)
+            assert lib.ma_biquad_set_state(h, vp(z0)) == 0
+            assert lib.ma_biquad_process_dev(h, ctypes.c_void_p(tin.pointer), length, ctypes.c_void_p(tout.pointer), length, length) == 0
+            device.synchronize()
+            assert max(o64.rel_rms(a, b) for a, b in zip(tout.toArray(), ref)) <= TOL
+            z = np.empty_like(z0)
+            assert lib.ma_biquad_get_state(h, vp(z)) == 0
+            assert np.max(np.abs(z - zref)) <= 1e-4 * max(1.0, float(np.max(np.abs(zref))))
+    finally:
+        lib.ma_biquad_destroy(h)
