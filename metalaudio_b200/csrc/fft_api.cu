@@ -82,7 +82,7 @@ ma_status ma_fft_plan_create(ma_context* ctx, int32_t n, const float* window, in
         if (!syn.empty()) st = upload(ctx, syn.data(), syn.size() * sizeof(float), (void**)&p->d_window_syn);
     }
     if (st == MA_OK && !p->large) {
-        cudaError_t e = cudaMalloc((void**)&p->d_norm, 2 * sizeof(float) * (size_t)hop);
+        cudaError_t e = cudaMalloc((void**)&p->d_norm, 2 * sizeof(float) * ((size_t)hop + (size_t)n));
         if (e != cudaSuccess) st = cuda_fail(e);
     }
     if (st == MA_OK && !p->large) {

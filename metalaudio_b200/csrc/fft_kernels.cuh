@@ -384,6 +384,8 @@ struct C2RParams {
     float* tail;                // streaming convolution step: per-signal overlap tail (N/2 floats)
     const float* norm_mid;      // iSTFT: clamped window sums of the interior, indexed by position mod hop
     const float* norm_mid_inv;  // iSTFT: their reciprocals
+    const float* norm_edge;     // iSTFT: window sums of the first N positions, then of the last frame's N positions
+                                // (host_tables.h make_edge_tables), or nullptr
     int32_t* error_flag;        // set to 1 when a bounded wait ran out
     int32_t dependent_launch;   // launched with programmatic stream serialization (see fft_small.cu)
     const float4* window_syn;   // register-ring iSTFT: synthesis window in thread order with 1/N folded in
@@ -752,6 +754,16 @@ MA_HD float window_sum_at(const float* __restrict__ window, int64_t o, int N, in
     return acc > floor ? acc : floor;
 }
 
+// The same for a position near an end of the signal (o < N - hop, or completed by the last frame).  With more frames than overlap
+// one another those positions see only one end of the signal, and their sums are tabulated: evaluated in
+// place they cost two 64-bit divisions and a chain of loads per sample, which made the CTAs that hold a
+// signal's ends the ones every short batch waited for (8 signals of 332 frames, 4096 points, hop 1024: 69 -> 49 us).
+MA_HD float window_sum_edge(const C2RParams& p, int64_t o, int N, int hop, int64_t frames) {
+    if (p.norm_edge != nullptr && (frames - 1) * hop >= (int64_t)(N - hop))
+        return o < (frames - 1) * (int64_t)hop ? MA_LDG(p.norm_edge + o) : MA_LDG(p.norm_edge + N + (o - (frames - 1) * hop));
+    return window_sum_at(p.window, o, N, hop, frames, p.floor);
+}
+
 // iSTFT: one CTA (T threads, one frame at a time) owns the frames [f0, f1) of one signal
 // and the output samples [f0*hop, f1*hop) (through the end of the signal for the last
 // chunk).  Overlap-add runs in a shared-memory ring of N floats; the frames before f0 that
@@ -838,7 +850,7 @@ MA_HD void istft_body(const C2RParams& p, Cta& cta, float2* smem) {
                     if (normalise) {
                         // interior positions (all overlapping frames exist) share hop distinct sums
                         const bool mid = o >= (int64_t)(N - hop) && o < F * (int64_t)hop;
-                        const float ws = mid ? MA_LDG(p.norm_mid + i) : window_sum_at(p.window, o, N, hop, F, p.floor);
+                        const float ws = mid ? MA_LDG(p.norm_mid + i) : window_sum_edge(p, o, N, hop, F);
                         r = acc / ws;
                     }
                     p.out[s * p.out_signal_stride + o] = r;
@@ -846,6 +858,106 @@ MA_HD void istft_body(const C2RParams& p, Cta& cta, float2* smem) {
             }
             cta.sync();
         }
+    }
+}
+
+// iSTFT of short frames (several fit a CTA) at any hop.  istft_body gives a frame to a CTA of its own, which
+// below 1024 points is less than one full warp.  Here the CTA's slots transform consecutive frames
+// side by side and leave the windowed samples in a ring of rows in shared memory; then all threads
+// add up, per output position, the rows that cover it (in frame order, as everywhere) and store the
+// completed samples contiguously.  A CTA owns a contiguous range of the global frame list like
+// istft_fast_body and rebuilds the `reach` frames in front of it.
+// smem: two exchange buffers | rows [FPC + reach][N] floats.
+template <int M, int LAYOUT, class Cta>
+MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
+    using P = FftPlan<M>;
+    using S = CtaShape<M>;
+    constexpr int R = P::R, T = P::T, N = 2 * M, FPC = S::FPC;
+    const int tid = cta.tid();
+    const int slot = tid / T;
+    const int t = tid % T;
+    float2* sbuf0 = smem + slot * S::ELEMS;
+    float* rows = reinterpret_cast<float*>(smem + 2 * S::BUF_STRIDE);
+    int parity = 0;
+    const float scale = 1.0f / (float)N;
+    const int hop = p.hop;
+    const int64_t F = p.frames_per_signal;
+    const bool normalise = !(p.window == nullptr && p.floor < 0.f);
+    const int reach = (N + hop - 1) / hop - 1;
+    const int n_rows = FPC + reach;
+    const int k_full = (N - 1) / hop, r_full = (N - 1) - k_full * hop;  // frames covering offset r: k_full + (r <= r_full)
+
+    float2 wreg[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+        const int n = t + q * T;
+        if (p.window != nullptr)
+            wreg[q] = make_float2(MA_LDG(p.window + 2 * n) * scale, MA_LDG(p.window + 2 * n + 1) * scale);
+        else
+            wreg[q] = make_float2(scale, scale);
+    }
+    const int64_t total = p.n_signals * F;
+    const int64_t per = (total + cta.nblocks() - 1) / cta.nblocks();
+    int64_t G = (int64_t)cta.bid() * per;
+    const int64_t G1 = G + per < total ? G + per : total;
+    while (G < G1) {  // one signal's part of the range at a time
+        const int64_t s = G / F;
+        const int64_t f0 = G - s * F;
+        const int64_t f1 = f0 + (G1 - G) < F ? f0 + (G1 - G) : F;
+        G += f1 - f0;
+        float* out = p.out + s * p.out_signal_stride;
+        int base = 0;  // row of frame fb
+        for (int64_t fb = f0 > reach ? f0 - reach : 0; fb < f1; fb += FPC) {
+            const int nb = f1 - fb < FPC ? (int)(f1 - fb) : FPC;
+            const int64_t f = fb + slot;
+            float2 v[R];
+            c2r_frame<M, LAYOUT, false, Cta>(p, slot < nb, s, f, s * F + f, t, sbuf0, S::BUF_STRIDE, parity, v, cta);
+            if (slot < nb) {
+                int row = base + slot;
+                if (row >= n_rows) row -= n_rows;
+                float2* dst = reinterpret_cast<float2*>(rows + row * N);
+#pragma unroll
+                for (int q = 0; q < R; ++q) dst[t + q * T] = make_float2(v[q].y * wreg[q].x, v[q].x * wreg[q].y);
+            }
+            cta.sync();
+            // positions the frames of this batch complete, counted from frame fb's start
+            const int first = fb < f0 ? (f0 - fb < nb ? (int)(f0 - fb) : nb) : 0;
+            const int64_t start = fb * (int64_t)hop;
+            int end = fb + nb == F ? (nb - 1) * hop + N : nb * hop;
+            if (start + end > p.out_len) end = (int)(p.out_len - start);
+            int i = first * hop + tid;
+            int j = i / hop, r = i - j * hop;
+            for (; i < end; i += S::THREADS) {
+                // frames fb + j - k, k = most .. least, cover the position at offset r + k*hop
+                int most = r <= r_full ? k_full : k_full - 1;
+                if (most > fb + j) most = (int)(fb + j);
+                const int least = j >= nb ? j - (nb - 1) : 0;
+                float acc = 0.f;
+                int row = base + j - most;
+                if (row < 0) row += n_rows;
+                else if (row >= n_rows) row -= n_rows;
+                for (int k = most; k >= least; --k) {
+                    acc += rows[row * N + r + k * hop];
+                    if (++row == n_rows) row = 0;
+                }
+                if (normalise) {
+                    const int64_t o = start + i;
+                    // interior positions (all overlapping frames exist) share hop distinct sums
+                    if (o >= (int64_t)(N - hop) && o < F * (int64_t)hop) acc *= MA_LDG(p.norm_mid_inv + r);
+                    else acc = acc / window_sum_edge(p, o, N, hop, F);
+                }
+                out[start + i] = acc;
+                r += S::THREADS;
+                while (r >= hop) {
+                    r -= hop;
+                    ++j;
+                }
+            }
+            base += FPC;
+            if (base >= n_rows) base -= n_rows;
+            // the next batch's rows are written behind at least one barrier of its transform
+        }
+        cta.sync();  // another signal (or another start) lays the rows out afresh
     }
 }
 
@@ -1121,8 +1233,8 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
                                 r2.y *= inv.y;
                             } else {
                                 const int64_t o = start + i0;
-                                r2.x = r2.x / window_sum_at(p.window, o, N, hop, F, p.floor);
-                                r2.y = r2.y / window_sum_at(p.window, o + 1, N, hop, F, p.floor);
+                                r2.x = r2.x / window_sum_edge(p, o, N, hop, F);
+                                r2.y = r2.y / window_sum_edge(p, o + 1, N, hop, F);
                             }
                         }
                         store_pair_before(out + i0, r2, p.out_len - (start + i0));
@@ -1153,8 +1265,8 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
                             r2.y = acc.y * inv.y;
                         } else {
                             const int64_t o = start + i0;
-                            r2.x = acc.x / window_sum_at(p.window, o, N, hop, F, p.floor);
-                            r2.y = acc.y / window_sum_at(p.window, o + 1, N, hop, F, p.floor);
+                            r2.x = acc.x / window_sum_edge(p, o, N, hop, F);
+                            r2.y = acc.y / window_sum_edge(p, o + 1, N, hop, F);
                         }
                     }
                     store_pair_before(out + i0, r2, p.out_len - (start + i0));

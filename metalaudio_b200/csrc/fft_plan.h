@@ -17,7 +17,8 @@ struct ma_fft_plan {
     float2* d_twInv = nullptr;  // stage tables the inverse kernels use (reversed order when pairable)
     float2* d_twN = nullptr;    // small path: exp(-2 pi i k/N), k <= M/2
     std::vector<float> h_window;  // host copy of the window (empty: none)
-    float* d_norm = nullptr;    // iSTFT interior normaliser, hop floats (see launch_istft_small)
+    float* d_norm = nullptr;    // iSTFT window sums: interior and its reciprocals (hop floats each), edges (2N floats)
+    int rows_occ[2] = {0, 0};   // resident CTAs per SM of the row-ring iSTFT at this hop (half interleaved, other layouts)
     float norm_floor = -1.0f;   // floor the table was built for
     // large path (N = n1 * n2): see fft_large.cu
     int n1 = 0, n2 = 0;

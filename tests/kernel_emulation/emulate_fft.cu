@@ -89,6 +89,8 @@ int emul_istft(int n, int hop, const float* in_a, const float* in_b, long long i
     for (int r = 0; r < hop; ++r) norm[(size_t)(hop + r)] = 1.0f / norm[(size_t)r];
     p.norm_mid = norm.data();
     p.norm_mid_inv = norm.data() + hop;
+    const auto edge = make_edge_tables(window, n, hop, floor);
+    p.norm_edge = edge.data();
     auto syn = make_synthesis_table(window, M);
     p.window_syn = (window != nullptr && !syn.empty()) ? reinterpret_cast<const float4*>(syn.data()) : nullptr;
     p.twM = twM.data(); p.twN = twN.data();
@@ -146,6 +148,45 @@ int emul_conv_blocks(int n, const float* in, long long signal_stride, long long 
         }
     };
 #define RUN(MM) run(std::integral_constant<int, MM>{});
+    MA_DISPATCH_M(M, RUN)
+#undef RUN
+    return rc;
+}
+
+// The short-frame iSTFT with its ring of rows; -1 for lengths whose CTAs hold a single frame.
+int emul_istft_rows(int n, int hop, const float* in_a, const float* in_b, long long frames, long long n_signals, int layout,
+                    const float* window, float floor, float* out, long long out_signal_stride, long long out_len, int nblocks) {
+    const int M = n / 2;
+    auto twM = make_stage_tables_for(M, plan_pairable_rt(M));
+    auto twN = make_hermitian_table(M);
+    C2RParams p{};
+    p.in_a = in_a; p.in_b = in_b; p.in_frame_stride = layout == LAYOUT_HALF_PACKED ? M : M + 1;
+    p.in_signal_stride = frames * p.in_frame_stride;
+    p.frames_per_signal = frames; p.n_signals = n_signals; p.layout = layout; p.hop = hop;
+    p.window = window; p.out = out; p.out_signal_stride = out_signal_stride; p.out_len = out_len; p.floor = floor;
+    std::vector<float> norm(2 * (size_t)hop, 1.f);
+    if (!(window == nullptr && floor < 0.f)) {
+        norm = make_norm_table(window, n, hop, floor);
+        norm.resize(2 * (size_t)hop);
+        for (int r = 0; r < hop; ++r) norm[(size_t)(hop + r)] = 1.0f / norm[(size_t)r];
+    }
+    p.norm_mid = norm.data();
+    p.norm_mid_inv = norm.data() + hop;
+    const auto edge = make_edge_tables(window, n, hop, floor);
+    p.norm_edge = edge.data();
+    p.twM = twM.data(); p.twN = twN.data();
+    int rc = -1;
+#define RUN(MM)                                                                              \
+    if constexpr (CtaShape<MM>::FPC > 1) {                                                   \
+        using S = CtaShape<MM>;                                                              \
+        const int reach = (n + hop - 1) / hop - 1;                                           \
+        const size_t smem = 2 * S::BUF_STRIDE * sizeof(float2) + (size_t)(S::FPC + reach) * n * sizeof(float); \
+        run_grid(nblocks, S::THREADS, smem, [&](HostCta& cta, void* sm) {                    \
+            if (layout == 0) istft_rows_body<MM, 0, HostCta>(p, cta, (float2*)sm);           \
+            else istft_rows_body<MM, -1, HostCta>(p, cta, (float2*)sm);                      \
+        });                                                                                  \
+        rc = 0;                                                                              \
+    }
     MA_DISPATCH_M(M, RUN)
 #undef RUN
     return rc;

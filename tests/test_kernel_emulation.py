@@ -42,6 +42,8 @@ def emul():
     lib.emul_istft.argtypes = [ctypes.c_int, ctypes.c_int, FP, FP, LL, LL, LL, LL, ctypes.c_int, FP, ctypes.c_float,
                                FP, LL, LL, ctypes.c_int, ctypes.c_int]
     lib.emul_conv_blocks.argtypes = [ctypes.c_int, FP, LL, LL, LL, LL, ctypes.c_int, FP, FP, LL, LL, ctypes.c_int]
+    lib.emul_istft_rows.argtypes = [ctypes.c_int, ctypes.c_int, FP, FP, LL, LL, ctypes.c_int, FP, ctypes.c_float, FP, LL, LL,
+                                    ctypes.c_int]
     lib.emul_tiled_rows.argtypes = [ctypes.c_int, LL, ctypes.POINTER(LL)]
     lib.emul_tiled_rows.restype = LL
     return lib
@@ -143,6 +145,36 @@ def test_convolution_block_transforms(emul, n, length_off, stride_mod, cut):
         assert o64.rel_rms(spec[..., 1:, 0] + 1j * spec[..., 1:, 1], ref[..., 1:b]) <= 1e-6
         assert np.allclose(spec[..., 0, 1], ref[..., b].real, atol=1e-3)
         assert o64.rel_rms(y, tail[:, :out_len]) <= 1e-6
+
+
+@pytest.mark.parametrize("n,hop", [(512, 160), (512, 512), (512, 511), (256, 64), (64, 7), (16, 1), (1024, 320), (4, 3), (2, 1)])
+@pytest.mark.parametrize("frames,signals,nblocks", [(1, 1, 1), (5, 3, 4), (37, 2, 3), (40, 2, 7)])
+@pytest.mark.parametrize("layout,cut", [(0, 0), (2, 0), (2, 3)])
+def test_short_frame_istft_rows(emul, n, hop, frames, signals, nblocks, layout, cut):
+    """The short-frame iSTFT: batches of frames in a ring of rows, ranges that start inside a signal and
+    run into the next one, hops that do not divide the frame, rows that end inside the last frame."""
+    cut = min(cut, hop - 1, (frames - 1) * hop + n - 1)
+    out_len = (frames - 1) * hop + n - cut
+    stride = out_len + 5
+    rng = np.random.default_rng(n + hop + frames)
+    w = rp.window("hamming", n) if n > 2 else np.ones(n, np.float32)
+    x = rng.standard_normal((signals, frames, n)).astype(np.float32)
+    spec = np.fft.rfft(x, axis=-1).astype(np.complex64)
+    if layout == 2:
+        packed = spec[..., :-1].copy()
+        packed[..., 0] = spec[..., 0].real + 1j * spec[..., -1].real
+        spec = packed
+    spec = np.ascontiguousarray(spec).view(np.float32)
+    y = np.full((signals, stride), 7.0, np.float32)
+    assert emul.emul_istft_rows(n, hop, fp(spec), None, frames, signals, layout, fp(w), 1e-8, fp(y), stride, out_len, nblocks) == 0
+    assert np.all(y[:, out_len:] == 7.0)
+    full = (frames - 1) * hop + n
+    ref, ws = np.zeros((signals, full)), np.zeros(full)
+    w64 = w.astype(np.float64)
+    for k in range(frames):
+        ref[:, k * hop:k * hop + n] += x[:, k] * w64
+        ws[k * hop:k * hop + n] += w64 ** 2
+    assert o64.rel_rms(y[:, :out_len], (ref / np.maximum(ws, 1e-8))[:, :out_len]) <= 1e-5
 
 
 @pytest.mark.parametrize("n,cut", [(256, 1), (256, 130), (256, 200), (1024, 777), (4096, 4000)])
