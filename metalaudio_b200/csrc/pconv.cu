@@ -238,6 +238,8 @@ __global__ void __launch_bounds__(kMacThreads) pconv_mac_kernel(const MacParams 
 // rows in a ring of 128 rows (each row enters once per CTA), the partition rows double-buffered.
 // That leaves about 0.25 byte of L2 traffic per complex multiply-accumulate and makes the FMA
 // pipe the limiter.  One barrier per chunk (1024 FMAs per thread apart).
+// A complex product is two packed two-wide multiply-adds, on the window row and on its swapped copy (64 partitions
+// of 2048 bins, 512 channels x 576 blocks: 7.50 -> 7.13 ms against four scalar ones).
 // TWO_LEVEL: every kFlushChunks chunks the running sums are added into a second set of
 // accumulators and cleared, so no float32 sum runs over more than TT*kFlushChunks partitions
 // (blocked summation: the rounding error of thousands of partitions grows with the block
@@ -287,13 +289,14 @@ __global__ void __launch_bounds__(128) pconv_mac_tiled_kernel(const MacParams q,
     __pipeline_wait_prior(0);
     __syncthreads();
 
-    float2 acc[TT], xw[TT];
+    float2 acc[TT], xw[TT], xs_[TT];  // window rows as (re, im) and as (im, re)
     float2 acc2[TWO_LEVEL ? TT : 1];
 #pragma unroll
     for (int i = 0; i < TT; ++i) {
         acc[i] = make_float2(0.f, 0.f);
         if constexpr (TWO_LEVEL) acc2[i] = make_float2(0.f, 0.f);
         xw[i] = xs[(base + i) & (RING - 1)][lane];
+        xs_[i] = make_float2(xw[i].y, xw[i].x);
     }
     int buf = 0;
     int since_flush = 0;
@@ -312,17 +315,18 @@ __global__ void __launch_bounds__(128) pconv_mac_tiled_kernel(const MacParams q,
                 const int p = p0 + j;
                 if (FULL || p < P) {
                     // slot (i - j) mod TT holds timeline row base + i - p; the row base - p enters at i = 0
-                    if (j > 0 || p0 > 0) xw[(TT - j) % TT] = xs[(base - p) & (RING - 1)][lane];
+                    if (j > 0 || p0 > 0) {
+                        const float2 x = xs[(base - p) & (RING - 1)][lane];
+                        xw[(TT - j) % TT] = x;
+                        xs_[(TT - j) % TT] = make_float2(x.y, x.x);
+                    }
                     const float2 h = hrow[j * 32];
                     const float ha = dc ? 0.f : h.y;   // bin 0 carries (DC, Nyquist): component-wise product
-                    const float hb = dc ? h.y : h.x;
+                    const float2 h1 = make_float2(h.x, dc ? h.y : h.x), h2 = make_float2(-ha, ha);
 #pragma unroll
                     for (int i = 0; i < TT; ++i) {
-                        const float2 xv = xw[(i - j + TT) % TT];
-                        acc[i].x = fmaf(xv.x, h.x, acc[i].x);
-                        acc[i].x = fmaf(-xv.y, ha, acc[i].x);
-                        acc[i].y = fmaf(xv.x, ha, acc[i].y);
-                        acc[i].y = fmaf(xv.y, hb, acc[i].y);
+                        acc[i] = pfma(xw[(i - j + TT) % TT], h1, acc[i]);
+                        acc[i] = pfma(xs_[(i - j + TT) % TT], h2, acc[i]);
                     }
                 }
             }

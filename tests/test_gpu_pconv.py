@@ -188,7 +188,7 @@ def test_whole_signal_writes_only_its_rows(device, lib, block, taps, length):
         assert o64.rel_rms(y[i * full:(i + 1) * full], o64.convolve_full(x[i], h)) <= TOL
 
 
-@pytest.mark.parametrize("block,taps", [(64, 1023), (64, 1024), (128, 2048), (64, 40001), (256, 33000), (2048, 40000)])
+@pytest.mark.parametrize("block,taps", [(64, 1023), (64, 1024), (128, 2048), (64, 9001), (256, 33000)])
 def test_whole_signal_after_steps_and_back(device, lib, block, taps):
     """Whole-signal calls on a clear delay line run on a coarser partition (from 16 partitions up); a call that
     follows streaming steps continues with their history on the caller's block size, and the calls and
