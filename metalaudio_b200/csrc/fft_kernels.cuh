@@ -174,8 +174,12 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
     float2* sbuf0 = smem + slot * S::ELEMS;
     int parity = 0;
 
+    // Kernels without staging read the window per frame through L1: its registers are worth a fifth CTA per SM
+    // (512 signals x 1017 frames of 512 points at odd row starts: 511 -> 401 us).
+    constexpr bool WREG = !HALF && ALIGNED && LAYOUT >= 0 && plan_pairable<M>();
+    const float2* window2 = reinterpret_cast<const float2*>(p.window);
     float2 wreg[R];
-    if (!HALF && p.window != nullptr) {
+    if (WREG && p.window != nullptr) {
 #pragma unroll
         for (int q = 0; q < R; ++q) {
             const int n = t + q * T;
@@ -281,17 +285,24 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
                 const int n = t + q * T;
                 float2 x = make_float2(0.f, 0.f);
                 if (active) x = MA_LDG(reinterpret_cast<const float2*>(src) + n);
-                v[q] = make_float2(x.x * wreg[q].x, x.y * wreg[q].y);
+                if (WREG) {
+                    v[q] = make_float2(x.x * wreg[q].x, x.y * wreg[q].y);
+                } else {
+                    const float2 w = p.window != nullptr ? MA_LDG(window2 + n) : make_float2(1.f, 1.f);
+                    v[q] = make_float2(x.x * w.x, x.y * w.y);
+                }
             }
         } else {
+            const int64_t left = p.signal_len - start;
+            const int valid = !active ? 0 : left < p.frame_valid ? (int)left : p.frame_valid;  // samples that exist
 #pragma unroll
             for (int q = 0; q < R; ++q) {
                 const int i0 = 2 * (t + q * T);
                 float x0 = 0.f, x1 = 0.f;
-                if (active && i0 < p.frame_valid && start + i0 < p.signal_len) x0 = MA_LDG(src + i0);
-                if (active && i0 + 1 < p.frame_valid && start + i0 + 1 < p.signal_len)
-                    x1 = MA_LDG(src + i0 + 1);
-                v[q] = make_float2(x0 * wreg[q].x, x1 * wreg[q].y);
+                if (i0 < valid) x0 = MA_LDG(src + i0);
+                if (i0 + 1 < valid) x1 = MA_LDG(src + i0 + 1);
+                const float2 w = p.window != nullptr ? MA_LDG(window2 + (t + q * T)) : make_float2(1.f, 1.f);
+                v[q] = make_float2(x0 * w.x, x1 * w.y);
             }
         }
 
@@ -567,7 +578,7 @@ MA_HD void c2r_frame(const C2RParams& p, bool active, int64_t s, int64_t f, int6
         }
         fft_run<PR, 1, true, false, Cta, TWALU, Hook, SINGLE, TWS1>(v, t, sbuf0, buf_stride, parity, p.twM, cta, twb, hook, tw_s1);
     } else {
-        float2* sb = sbuf0 + parity * buf_stride;
+        float2* sb = SINGLE ? sbuf0 : sbuf0 + parity * buf_stride;
         parity ^= 1;
         // All loads first (one memory round trip per partial spectrum, not one per bin), then the
         // arithmetic.
@@ -606,6 +617,7 @@ MA_HD void c2r_frame(const C2RParams& p, bool active, int64_t s, int64_t f, int6
                 pa[0] = make_float2(pa[0].x, 0.f);
             }
         }
+        if constexpr (SINGLE) cta.sync();  // the previous exchange's reads are done
 #pragma unroll
         for (int q = 0; q <= R / 2; ++q) {
             const int k = t + q * T;
@@ -619,7 +631,7 @@ MA_HD void c2r_frame(const C2RParams& p, bool active, int64_t s, int64_t f, int6
         cta.sync();
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = sb[saddr<1>(t + q * T)];
-        fft_forward_regs<M, 1, Cta>(v, t, sbuf0, buf_stride, parity, p.twM, cta);
+        fft_forward_regs<M, 1, Cta, SINGLE>(v, t, sbuf0, buf_stride, parity, p.twM, cta);
     }
 }
 
@@ -867,7 +879,9 @@ MA_HD void istft_body(const C2RParams& p, Cta& cta, float2* smem) {
 // add up, per output position, the rows that cover it (in frame order, as everywhere) and store the
 // completed samples contiguously.  A CTA owns a contiguous range of the global frame list like
 // istft_fast_body and rebuilds the `reach` frames in front of it.
-// smem: two exchange buffers | rows [FPC + reach][N] floats.
+// smem: exchange buffer | window times 1/N [N] floats | rows [FPC + reach][N] floats.  One exchange buffer and the
+// window out of the registers make room for five CTAs of 128 threads per SM instead of three: the kernel waits for
+// latencies, not for a pipe (512 signals x 1017 frames of 512 points, hop 160: 880 -> 737 us).
 template <int M, int LAYOUT, class Cta>
 MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
     using P = FftPlan<M>;
@@ -877,7 +891,8 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
     const int slot = tid / T;
     const int t = tid % T;
     float2* sbuf0 = smem + slot * S::ELEMS;
-    float* rows = reinterpret_cast<float*>(smem + 2 * S::BUF_STRIDE);
+    float2* wtab = smem + S::BUF_STRIDE;
+    float* rows = reinterpret_cast<float*>(wtab + M);
     int parity = 0;
     const float scale = 1.0f / (float)N;
     const int hop = p.hop;
@@ -887,15 +902,9 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
     const int n_rows = FPC + reach;
     const int k_full = (N - 1) / hop, r_full = (N - 1) - k_full * hop;  // frames covering offset r: k_full + (r <= r_full)
 
-    float2 wreg[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-        const int n = t + q * T;
-        if (p.window != nullptr)
-            wreg[q] = make_float2(MA_LDG(p.window + 2 * n) * scale, MA_LDG(p.window + 2 * n + 1) * scale);
-        else
-            wreg[q] = make_float2(scale, scale);
-    }
+    for (int n = tid; n < M; n += S::THREADS)  // read behind the first batch's barriers
+        wtab[n] = p.window != nullptr ? make_float2(MA_LDG(p.window + 2 * n) * scale, MA_LDG(p.window + 2 * n + 1) * scale)
+                                      : make_float2(scale, scale);
     const int64_t total = p.n_signals * F;
     const int64_t per = (total + cta.nblocks() - 1) / cta.nblocks();
     int64_t G = (int64_t)cta.bid() * per;
@@ -911,13 +920,16 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
             const int nb = f1 - fb < FPC ? (int)(f1 - fb) : FPC;
             const int64_t f = fb + slot;
             float2 v[R];
-            c2r_frame<M, LAYOUT, false, Cta>(p, slot < nb, s, f, s * F + f, t, sbuf0, S::BUF_STRIDE, parity, v, cta);
+            c2r_frame<M, LAYOUT, false, Cta, false, NoHook, true>(p, slot < nb, s, f, s * F + f, t, sbuf0, S::BUF_STRIDE, parity, v, cta);
             if (slot < nb) {
                 int row = base + slot;
                 if (row >= n_rows) row -= n_rows;
                 float2* dst = reinterpret_cast<float2*>(rows + row * N);
 #pragma unroll
-                for (int q = 0; q < R; ++q) dst[t + q * T] = make_float2(v[q].y * wreg[q].x, v[q].x * wreg[q].y);
+                for (int q = 0; q < R; ++q) {
+                    const float2 w = wtab[t + q * T];
+                    dst[t + q * T] = make_float2(v[q].y * w.x, v[q].x * w.y);
+                }
             }
             cta.sync();
             // positions the frames of this batch complete, counted from frame fb's start

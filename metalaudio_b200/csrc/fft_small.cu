@@ -53,8 +53,14 @@ static void launch_maybe_dependent(K kernel, int grid, int threads, size_t smem,
     (void)cudaLaunchKernelEx(&cfg, kernel, p);  // an error is picked up by after_launch
 }
 
+// Kernels of several frames per CTA with a fixed layout but no staging fit five CTAs of 128 threads on an SM.
+template <int M, int LAYOUT>
+constexpr int r2c_ctas() {
+    return CtaShape<M>::FPC > 1 && LAYOUT >= 0 && !plan_pairable<M>() ? 5 : 512 / CtaShape<M>::THREADS;
+}
+
 template <int M, bool ALIGNED, int LAYOUT, int MAGK, bool HALF>
-__global__ void __launch_bounds__(CtaShape<M>::THREADS, 512 / CtaShape<M>::THREADS) r2c_kernel(const R2CParams p) {
+__global__ void __launch_bounds__(CtaShape<M>::THREADS, r2c_ctas<M, LAYOUT>()) r2c_kernel(const R2CParams p) {
     DevCta cta;
     if (p.dependent_launch) dependents_launch();
     r2c_body<M, ALIGNED, LAYOUT, MAGK, DevCta, HALF>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
@@ -86,7 +92,7 @@ istft_fast_kernel(const C2RParams p) {
 }
 
 template <int M, int LAYOUT>
-__global__ void __launch_bounds__(CtaShape<M>::THREADS, 512 / CtaShape<M>::THREADS) istft_rows_kernel(const C2RParams p) {
+__global__ void __launch_bounds__(CtaShape<M>::THREADS, CtaShape<M>::THREADS == 128 ? 5 : 1) istft_rows_kernel(const C2RParams p) {
     DevCta cta;
     istft_rows_body<M, LAYOUT, DevCta>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
 }
@@ -138,6 +144,11 @@ static ma_status launch_r2c_variant(ma_fft_plan* plan, const R2CParams& p, bool 
         // the convolution's zero-padded blocks
         if (!aligned && magk == -1 && p.layout == LAYOUT_HALF_PACKED && p.frame_valid == M && p.window == nullptr)
             return launch_r2c_t<M, true, LAYOUT_HALF_PACKED, -1, true>(plan, p);
+    }
+    if constexpr (!plan_pairable<M>() && M >= 64) {
+        if (p.layout == LAYOUT_HALF_INTERLEAVED && magk == -1)
+            return aligned ? launch_r2c_t<M, true, LAYOUT_HALF_INTERLEAVED, -1>(plan, p)
+                           : launch_r2c_t<M, false, LAYOUT_HALF_INTERLEAVED, -1>(plan, p);
     }
     return aligned ? launch_r2c_t<M, true, -1, -2>(plan, p) : launch_r2c_t<M, false, -1, -2>(plan, p);
 }
@@ -215,7 +226,7 @@ template <int M>
 static size_t istft_rows_smem(int hop) {
     using S = CtaShape<M>;
     const int reach = (2 * M + hop - 1) / hop - 1;
-    return 2 * (size_t)S::BUF_STRIDE * sizeof(float2) + (size_t)(S::FPC + reach) * 2 * M * sizeof(float);
+    return ((size_t)S::BUF_STRIDE + M) * sizeof(float2) + (size_t)(S::FPC + reach) * 2 * M * sizeof(float);
 }
 
 // Short frames without a thread-private ring (see istft_rows_body).

@@ -180,7 +180,7 @@ int emul_istft_rows(int n, int hop, const float* in_a, const float* in_b, long l
     if constexpr (CtaShape<MM>::FPC > 1) {                                                   \
         using S = CtaShape<MM>;                                                              \
         const int reach = (n + hop - 1) / hop - 1;                                           \
-        const size_t smem = 2 * S::BUF_STRIDE * sizeof(float2) + (size_t)(S::FPC + reach) * n * sizeof(float); \
+        const size_t smem = (S::BUF_STRIDE + MM) * sizeof(float2) + (size_t)(S::FPC + reach) * n * sizeof(float); \
         run_grid(nblocks, S::THREADS, smem, [&](HostCta& cta, void* sm) {                    \
             if (layout == 0) istft_rows_body<MM, 0, HostCta>(p, cta, (float2*)sm);           \
             else istft_rows_body<MM, -1, HostCta>(p, cta, (float2*)sm);                      \
