@@ -211,18 +211,20 @@ struct Bfly {
 template <int M>
 struct FftPlan;
 
-#define MA_DEFINE_PLAN(M_, R_, NS_, R0, R1, R2)                                     \
-    template <>                                                                     \
-    struct FftPlan<M_> {                                                            \
+#define MA_PLAN_BODY(M_, R_, NS_, R0, R1, R2, R3)                                   \
+    {                                                                               \
         static constexpr int M = M_;                                                \
         static constexpr int R = R_;                                                \
         static constexpr int T = M_ / R_;                                           \
         static constexpr int NS = NS_;                                              \
-        static constexpr __host__ __device__ int radix(int s) { return s == 0 ? R0 : (s == 1 ? R1 : R2); } \
+        static constexpr __host__ __device__ int radix(int s) { return s == 0 ? R0 : (s == 1 ? R1 : (s == 2 ? R2 : R3)); } \
         static constexpr __host__ __device__ int ns_before(int s) {                                     \
-            return s == 0 ? 1 : (s == 1 ? R0 : R0 * R1);                            \
+            return s == 0 ? 1 : (s == 1 ? R0 : (s == 2 ? R0 * R1 : R0 * R1 * R2));  \
         }                                                                           \
     };
+#define MA_DEFINE_PLAN(M_, R_, NS_, R0, R1, R2) \
+    template <>                                 \
+    struct FftPlan<M_> MA_PLAN_BODY(M_, R_, NS_, R0, R1, R2, 1)
 
 MA_DEFINE_PLAN(1, 1, 1, 1, 1, 1)
 MA_DEFINE_PLAN(2, 2, 1, 2, 1, 1)
@@ -236,20 +238,32 @@ MA_DEFINE_PLAN(256, 16, 2, 16, 16, 1)
 MA_DEFINE_PLAN(512, 16, 3, 16, 8, 4)
 MA_DEFINE_PLAN(1024, 16, 3, 16, 8, 8)
 MA_DEFINE_PLAN(2048, 16, 3, 16, 16, 8)
-MA_DEFINE_PLAN(4096, 16, 3, 16, 16, 16)
+// Four stages, so that the last one has several butterflies per thread and the pairs k, M - k meet in one
+// thread: three exchanges, as 16*16*16 needs with the Hermitian one.  This order of the radices keeps the
+// exchanges free of bank conflicts in both directions.
+template <>
+struct FftPlan<4096> MA_PLAN_BODY(4096, 16, 4, 16, 4, 16, 4)
 #undef MA_DEFINE_PLAN
 
-// Threads per transform of the plan for length m (0 for a length without a plan).
+// Plans of the two-pass transforms' rows and columns, which are complex or bring their own Hermitian step:
+// the fewest exchanges.
+template <int M>
+struct LargePlan : FftPlan<M> {};
+template <>
+struct LargePlan<4096> MA_PLAN_BODY(4096, 16, 3, 16, 16, 16, 1)
+#undef MA_PLAN_BODY
+
+// Threads per transform of the two-pass transforms' plan for length m (0 for a length without a plan).
 inline int fft_plan_threads(int m) {
     switch (m) {
-        case 32: return FftPlan<32>::T;
-        case 64: return FftPlan<64>::T;
-        case 128: return FftPlan<128>::T;
-        case 256: return FftPlan<256>::T;
-        case 512: return FftPlan<512>::T;
-        case 1024: return FftPlan<1024>::T;
-        case 2048: return FftPlan<2048>::T;
-        case 4096: return FftPlan<4096>::T;
+        case 32: return LargePlan<32>::T;
+        case 64: return LargePlan<64>::T;
+        case 128: return LargePlan<128>::T;
+        case 256: return LargePlan<256>::T;
+        case 512: return LargePlan<512>::T;
+        case 1024: return LargePlan<1024>::T;
+        case 2048: return LargePlan<2048>::T;
+        case 4096: return LargePlan<4096>::T;
         default: return 0;
     }
 }
@@ -277,6 +291,13 @@ struct FftPlanRev {
 template <int M_>
 constexpr __host__ __device__ bool plan_pairable() {
     return FftPlan<M_>::NS >= 2 && (FftPlan<M_>::R / FftPlan<M_>::radix(FftPlan<M_>::NS - 1)) >= 2;
+}
+
+// Whether the paired kernels expand a stage's twiddles from one base per butterfly in registers.  The four-stage
+// plan reads the exact tables, as its length always did: a chain multiplies the base's rounding.
+template <int M_>
+constexpr __host__ __device__ bool plan_chains() {
+    return plan_pairable<M_>() && FftPlan<M_>::NS <= 3;
 }
 
 // Shared-memory addressing.  W == 1: one transform owns a contiguous region, element idx
@@ -547,10 +568,9 @@ MA_HD void fft_run(float2* v, int t, float2* sbuf0, int buf_stride, int& parity,
 // Complex forward FFT of length M in natural order.  In: v[q] = z[t + q*T].
 // Out: v[q] = Z[t + q*T].
 // SINGLE: one exchange buffer (buf_stride is ignored), a barrier in front of every exchange write.
-template <int M, int W, class Cta, bool SINGLE = false>
+template <int M, int W, class Cta, bool SINGLE = false, class P = FftPlan<M>>
 MA_HD void fft_forward_regs(float2* v, int t, float2* sbuf0, int buf_stride, int& parity,
                             const float2* __restrict__ twM, Cta& cta) {
-    using P = FftPlan<M>;
     constexpr int R = P::R;
     fft_run<P, W, false, false, Cta, false, NoHook, SINGLE>(v, t, sbuf0, buf_stride, parity, twM, cta);
     // After the last stage, element (b, k) of the flat array is Z[t + (b + k*NB)*T].

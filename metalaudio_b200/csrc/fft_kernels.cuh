@@ -197,7 +197,7 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
     // The convolution's transforms (HALF) read the exact twiddles from the tables instead: a power chain
     // multiplies the rounding of its base by the power, which there more than doubled the error of the whole
     // convolution (2.0e-7 -> 4.9e-7 relative; 1.38 instead of 1.60 ms per 512 channels of 512 blocks).
-    constexpr bool TWALU = BULK && !HALF;
+    constexpr bool TWALU = BULK && !HALF && plan_chains<M>();
     float2 twb[tw_base_count<P>()];
     float2 wherm[R / 2 + 1];
     (void)wherm;
@@ -654,7 +654,7 @@ MA_HD void c2r_body(const C2RParams& p, Cta& cta, float2* smem) {
     using P = FftPlan<M>;
     using S = CtaShape<M>;
     constexpr int R = P::R, T = P::T, N = 2 * M;
-    constexpr bool TWALU = LAYOUT >= 0 && plan_pairable<M>();
+    constexpr bool TWALU = LAYOUT >= 0 && plan_chains<M>();
     const int tid = cta.tid();
     const int slot = tid / T;
     const int t = tid % T;
@@ -673,7 +673,7 @@ MA_HD void c2r_body(const C2RParams& p, Cta& cta, float2* smem) {
     const int64_t df = stride_frames - ds * p.frames_per_signal;
     // Staged variant (half layouts of paired plans): the next frame's row is brought into shared
     // memory by one bulk asynchronous copy while this frame is transformed.
-    constexpr bool STAGED = TWALU && (LAYOUT == LAYOUT_HALF_INTERLEAVED || LAYOUT == LAYOUT_HALF_PACKED);
+    constexpr bool STAGED = plan_pairable<M>() && (LAYOUT == LAYOUT_HALF_INTERLEAVED || LAYOUT == LAYOUT_HALF_PACKED);
     float2* stage_slot = smem + 2 * S::BUF_STRIDE + slot * S::ROW;
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem + 2 * S::BUF_STRIDE + S::FPC * S::ROW) + 2 * slot;
     uint32_t phase = 0;
@@ -1165,12 +1165,12 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
             }
         };
         if constexpr (POLAR) {
-            c2r_frame<M, LAYOUT, true, Cta, true, decltype(issue_next), SH::EXCH == 1, true>(
+            c2r_frame<M, LAYOUT, plan_chains<M>(), Cta, true, decltype(issue_next), SH::EXCH == 1, true>(
                 p, true, s, f, G, t, smem, SH::ELEMS, parity, v, cta, twb, wherm, stage, issue_next, nullptr, tw1);
         } else {
             const StagedRow r = staged_row<M>(p, s, f);
             // PLAIN: exact twiddles, as in the convolution's forward transform (see r2c_body)
-            c2r_frame<M, LAYOUT, !PLAIN, Cta, true, decltype(issue_next), SH::EXCH == 1, true>(
+            c2r_frame<M, LAYOUT, !PLAIN && plan_chains<M>(), Cta, true, decltype(issue_next), SH::EXCH == 1, true>(
                 p, true, s, f, G, t, smem, SH::ELEMS, parity, v, cta, twb, wherm, stage + r.shift, issue_next, r.row, tw1);
         }
 

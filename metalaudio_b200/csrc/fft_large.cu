@@ -43,9 +43,9 @@ struct LargeParams {
     int n, n1, n2;
     int layout, mag_kind;
     float db_scale;
-    const float2* twM2;  // stage twiddle tables of FftPlan<M2>
+    const float2* twM2;  // stage twiddle tables of LargePlan<M2>
     const float2* twN2;  // exp(-2 pi i k/N2), k <= M2/2
-    const float2* tw1;   // stage twiddle tables of FftPlan<N1>
+    const float2* tw1;   // stage twiddle tables of LargePlan<N1>
     // Pass twiddles exp(-2 pi i n1 k2 / N) as geometric sequences in k2 (column pass) or n1 (row passes),
     // laid out so that a warp's loads are contiguous:
     const float2* twc;       // [T(M2) + 2][N1]: rows t < T: n1*t; row T: the step n1*T; row T+1: n1*M2
@@ -101,8 +101,8 @@ constexpr int kRowsMulBigCtas = 1;
 
 // ---------------------------------------------------------------- forward pass 1
 template <int M2, int W1>
-__global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 256 ? kColsR2cCtas : kBigCtas) cols_r2c_kernel(const LargeParams p) {
-    using P = FftPlan<M2>;
+__global__ void __launch_bounds__(W1* LargePlan<M2>::T, (W1 * LargePlan<M2>::T) <= 256 ? kColsR2cCtas : kBigCtas) cols_r2c_kernel(const LargeParams p) {
+    using P = LargePlan<M2>;
     constexpr int R = P::R, T = P::T;
     float2* smem = reinterpret_cast<float2*>(ma_large_smem);
     const int i = threadIdx.x % W1;
@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 2
         }
         int parity = 0;
         float2* sbuf0 = smem + i;
-        fft_forward_regs<M2, W1, DevCtaL, true>(v, t, sbuf0, 0, parity, p.twM2, cta);
+        fft_forward_regs<M2, W1, DevCtaL, true, P>(v, t, sbuf0, 0, parity, p.twM2, cta);
         float2* sb = sbuf0;
         cta.sync();  // the exchange's reads are done before the buffer is rewritten
 #pragma unroll
@@ -173,8 +173,8 @@ __global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 2
 // 16-byte aligned inputs without window and tiles of 16 or 32 columns.  Launched with
 // one CTA per tile (the grid-stride loop runs once).
 template <int M2, int W1>
-__global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 256 ? kColsR2cTmaCtas : kBigCtas) cols_r2c_tma_kernel(const LargeParams p, const __grid_constant__ CUtensorMap in_map) {
-    using P = FftPlan<M2>;
+__global__ void __launch_bounds__(W1* LargePlan<M2>::T, (W1 * LargePlan<M2>::T) <= 256 ? kColsR2cTmaCtas : kBigCtas) cols_r2c_tma_kernel(const LargeParams p, const __grid_constant__ CUtensorMap in_map) {
+    using P = LargePlan<M2>;
     constexpr int R = P::R, T = P::T;
     float2* smem = reinterpret_cast<float2*>(ma_large_smem);
     const int i = threadIdx.x % W1;
@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 2
         }
         int parity = 0;
         float2* sbuf0 = smem + i;
-        fft_forward_regs<M2, W1, DevCtaL, true>(v, t, sbuf0, 0, parity, p.twM2, cta);
+        fft_forward_regs<M2, W1, DevCtaL, true, P>(v, t, sbuf0, 0, parity, p.twM2, cta);
         float2* sb = sbuf0;
         cta.sync();  // the exchange's reads are done before the buffer is rewritten
 #pragma unroll
@@ -347,8 +347,8 @@ constexpr __host__ __device__ size_t rows_smem_bytes() {
 
 // ---------------------------------------------------------------- forward pass 2
 template <int N1, int W2>
-__global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 256 ? 4 : kBigCtas) rows_fwd_kernel(const LargeParams p) {
-    using P = FftPlan<N1>;
+__global__ void __launch_bounds__(W2* LargePlan<N1>::T, (W2 * LargePlan<N1>::T) <= 256 ? 4 : kBigCtas) rows_fwd_kernel(const LargeParams p) {
+    using P = LargePlan<N1>;
     constexpr int R = P::R, T = P::T;
     constexpr int ELEMS = smem_elems_per_fft<N1, 1>();
     constexpr int BUF = ELEMS * W2;
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 2
         for (int q = 0; q < R; ++q) v[q] = active ? smem[slot * N1 + t + q * T] : make_float2(0.f, 0.f);
         cta.sync();  // every thread has its points: the exchange buffer may be written
         int parity = 0;
-        fft_forward_regs<N1, 1, DevCtaL, true>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
+        fft_forward_regs<N1, 1, DevCtaL, true, P>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
         cta.sync();  // everyone is done with the exchange buffers: reuse them as the tile
         float2* tile = smem;  // [k1][W2+1]
 #pragma unroll
@@ -436,8 +436,8 @@ __device__ __forceinline__ float2 load_bin(const LargeParams& p, int64_t b, int6
 
 // ---------------------------------------------------------------- inverse pass A
 template <int N1, int W2>
-__global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 256 ? 4 : kBigCtas) rows_inv_kernel(const LargeParams p) {
-    using P = FftPlan<N1>;
+__global__ void __launch_bounds__(W2* LargePlan<N1>::T, (W2 * LargePlan<N1>::T) <= 256 ? 4 : kBigCtas) rows_inv_kernel(const LargeParams p) {
+    using P = LargePlan<N1>;
     constexpr int R = P::R, T = P::T;
     constexpr int ELEMS = smem_elems_per_fft<N1, 1>();
     constexpr int BUF = ELEMS * W2;
@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 2
         }
         cta.sync();
         int parity = 0;
-        fft_forward_regs<N1, 1, DevCtaL, true>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
+        fft_forward_regs<N1, 1, DevCtaL, true, P>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
         const int64_t g = g0 + slot;
         if (g < rows_total) {
             const int k2 = (int)(g % (m2 + 1));
@@ -539,8 +539,8 @@ __global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 2
 // never leaves the registers.  STORE_SPECTRUM: stop after the forward transform and write the row
 // to p.spec_rows (how the kernel's own spectrum is prepared).
 template <int N1, int W2, bool STORE_SPECTRUM>
-__global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 256 ? 3 : kRowsMulBigCtas) rows_mul_kernel(const LargeParams p) {
-    using P = FftPlan<N1>;
+__global__ void __launch_bounds__(W2* LargePlan<N1>::T, (W2 * LargePlan<N1>::T) <= 256 ? 3 : kRowsMulBigCtas) rows_mul_kernel(const LargeParams p) {
+    using P = LargePlan<N1>;
     constexpr int R = P::R, T = P::T;
     constexpr int ELEMS = smem_elems_per_fft<N1, 1>();
     constexpr int BUF = ELEMS * W2;
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 2
             for (int q = 0; q < R; ++q) h[q] = __ldg(hrow + t + q * T);
         }
         int parity = 0;
-        fft_forward_regs<N1, 1, DevCtaL, true>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
+        fft_forward_regs<N1, 1, DevCtaL, true, P>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
         if constexpr (STORE_SPECTRUM) {
             if (active) {
 #pragma unroll
@@ -579,7 +579,7 @@ __global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 2
                 v[q] = make_float2(y.y, y.x);  // swapped: the inverse runs as a forward transform
             }
             cta.sync();  // the first transform's exchange reads are done before the buffers are rewritten
-            fft_forward_regs<N1, 1, DevCtaL, true>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
+            fft_forward_regs<N1, 1, DevCtaL, true, P>(v, t, smem + slot * ELEMS, BUF, parity, p.tw1, cta);
             if (active) {
                 float2 wq[R];
                 geometric_twiddles<R>(wq, __ldg(p.twr + k2 * T + t), __ldg(p.twr_step + k2));
@@ -593,8 +593,8 @@ __global__ void __launch_bounds__(W2* FftPlan<N1>::T, (W2 * FftPlan<N1>::T) <= 2
 
 // ---------------------------------------------------------------- inverse pass B
 template <int M2, int W1>
-__global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 256 ? kColsC2rCtas : kBigCtas) cols_c2r_kernel(const LargeParams p) {
-    using P = FftPlan<M2>;
+__global__ void __launch_bounds__(W1* LargePlan<M2>::T, (W1 * LargePlan<M2>::T) <= 256 ? kColsC2rCtas : kBigCtas) cols_c2r_kernel(const LargeParams p) {
+    using P = LargePlan<M2>;
     constexpr int R = P::R, T = P::T;
     float2* smem = reinterpret_cast<float2*>(ma_large_smem);
     const int i = threadIdx.x % W1;
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 2
         float2 v[R];
 #pragma unroll
         for (int q = 0; q < R; ++q) v[q] = sb[saddr<W1>(t + q * T)];
-        fft_forward_regs<M2, W1, DevCtaL, true>(v, t, sbuf0, 0, parity, p.twM2, cta);
+        fft_forward_regs<M2, W1, DevCtaL, true, P>(v, t, sbuf0, 0, parity, p.twM2, cta);
         float* x = p.out_a + b * (int64_t)p.n + n1;
 #pragma unroll
         for (int q = 0; q < R; ++q) {
@@ -654,10 +654,10 @@ __global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 2
 // one thread), and the real output tile - N2 rows of W1 samples - is assembled in the same buffer and
 // stored as boxes.  For 16-byte aligned dense outputs and tiles of 32 columns; one tile per CTA.
 template <int M2, int W1>
-__global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 256 ? kColsC2rCtas : kBigCtas)
+__global__ void __launch_bounds__(W1* LargePlan<M2>::T, (W1 * LargePlan<M2>::T) <= 256 ? kColsC2rCtas : kBigCtas)
     cols_c2r_tma_kernel(const LargeParams p, const __grid_constant__ CUtensorMap scratch_map,
                         const __grid_constant__ CUtensorMap out_map) {
-    using P = FftPlan<M2>;
+    using P = LargePlan<M2>;
     constexpr int R = P::R, T = P::T;
     constexpr int ROWS = 2 * M2, BOX_ROWS = ROWS < 256 ? ROWS : 256;
     float2* smem = reinterpret_cast<float2*>(ma_large_smem);
@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(W1* FftPlan<M2>::T, (W1 * FftPlan<M2>::T) <= 2
     float2 v[R];
 #pragma unroll
     for (int q = 0; q < R; ++q) v[q] = sbuf0[saddr<W1>(t + q * T)];
-    fft_forward_regs<M2, W1, DevCtaL, true>(v, t, sbuf0, 0, parity, p.twM2, cta);
+    fft_forward_regs<M2, W1, DevCtaL, true, P>(v, t, sbuf0, 0, parity, p.twM2, cta);
     cta.sync();  // the last exchange's reads are done: the buffer becomes the output tile [N2][W1]
     float* tile = reinterpret_cast<float*>(smem);
 #pragma unroll
@@ -787,7 +787,7 @@ static bool input_tensor_map(const LargeParams& p, int box_floats, int box_rows,
 
 template <int M2, int W1>
 static ma_status run_cols(ma_fft_plan* plan, const LargeParams& p, bool inverse, cudaStream_t st) {
-    constexpr int threads = W1 * FftPlan<M2>::T;
+    constexpr int threads = W1 * LargePlan<M2>::T;
     constexpr size_t smem = (size_t)M2 * W1 * sizeof(float2);
     ma_context* ctx = plan->ctx;
     auto kf = cols_r2c_kernel<M2, W1>;
@@ -839,7 +839,7 @@ static ma_status run_cols(ma_fft_plan* plan, const LargeParams& p, bool inverse,
 
 template <int N1, int W2>
 static ma_status run_rows(ma_fft_plan* plan, const LargeParams& p, bool inverse, cudaStream_t st) {
-    constexpr int threads = W2 * FftPlan<N1>::T;
+    constexpr int threads = W2 * LargePlan<N1>::T;
     // the exchange buffer plus 16 bytes for the staging barrier of the forward pass
     constexpr size_t smem = rows_smem_bytes<N1, W2>() + 16;
     ma_context* ctx = plan->ctx;
@@ -883,7 +883,7 @@ static ma_status kernel_occupancy(K kernel, int threads, size_t smem, int* occ) 
 
 template <int N1, int W2>
 static ma_status run_rows_mul(ma_fft_plan* plan, const LargeParams& p, bool store_spectrum, cudaStream_t st) {
-    constexpr int threads = W2 * FftPlan<N1>::T;
+    constexpr int threads = W2 * LargePlan<N1>::T;
     constexpr size_t smem = rows_smem_bytes<N1, W2>();
     ma_context* ctx = plan->ctx;
     static int occ[2][64] = {};
@@ -948,10 +948,10 @@ ma_status large_plan_init(ma_fft_plan* plan) {
     plan->n1 = s.n1;
     plan->n2 = 2 * s.m2;
     {
-        auto tw = make_stage_tables_for(s.m2, false);  // column stage twiddles
+        auto tw = make_large_tables_for(s.m2);  // column stage twiddles
         MA_CUDA(cudaMalloc((void**)&plan->d_twM, tw.size() * sizeof(float2)));
         MA_TRY(copy_h2d(ctx, plan->d_twM, tw.data(), tw.size() * sizeof(float2)));
-        auto t1 = make_stage_tables_for(s.n1, false);  // row stage twiddles
+        auto t1 = make_large_tables_for(s.n1);  // row stage twiddles
         MA_CUDA(cudaMalloc((void**)&plan->d_tw1, t1.size() * sizeof(float2)));
         MA_TRY(copy_h2d(ctx, plan->d_tw1, t1.data(), t1.size() * sizeof(float2)));
     }

@@ -80,6 +80,15 @@ inline std::vector<float2> make_stage_tables_for(int m, bool rev) {
     return out;
 }
 
+// Stage tables of the two-pass transforms' plan for complex length m.
+inline std::vector<float2> make_large_tables_for(int m) {
+    std::vector<float2> out;
+#define MA_LARGE_CASE(MM) out = make_stage_tables<LargePlan<MM>>()
+    MA_DISPATCH_M(m, MA_LARGE_CASE)
+#undef MA_LARGE_CASE
+    return out;
+}
+
 // Twiddles of the Hermitian pre/post-process, exp(-2 pi i idx / (2m)).  Pairable plans index
 // them [k][j] -> idx = j + k*NL with NL = m / (last forward radix), j <= NL/2, so that the lanes
 // of a warp (consecutive j) load contiguously; other plans use idx = k, k <= m/2.

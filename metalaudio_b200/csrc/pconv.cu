@@ -505,8 +505,8 @@ __global__ void pconv_history_kernel(float2* __restrict__ ring, float2* __restri
     }
 }
 
-// Largest block of the whole-signal calls: 4096-point transforms, the longest with the paired plans.
-constexpr int kWholeBlock = 2048;
+// Largest block of the whole-signal calls: 8192-point transforms, the longest that fit shared memory.
+constexpr int kWholeBlock = 4096;
 constexpr int kWholePartitions = 8;
 
 static void free_signal_buffers(ma_pconv* pc) {
@@ -546,10 +546,10 @@ static void free_coarse(ma_pconv* pc) {
 
 // Block size of whole-signal calls.  The multiply-accumulate costs one complex product per output bin and
 // partition, i.e. it shrinks with the number of partitions, while the transforms' cost per sample hardly
-// depends on their length up to 4096 points.  The shorter sums also round less, which pays for the longer
+// depends on their length up to 8192 points.  The shorter sums also round less, which pays for the longer
 // transforms' rounding as long as there are sums to shorten: at least kWholePartitions partitions stay.
-// Measured, 512 channels x 2^20 samples, 131072 taps, block 256: 512 partitions 64.2 ms, error 4.4e-7; 64 partitions
-// of 2048 samples 15.2 ms (10.8 ms with the paired plans' block transforms), error 2.9e-7.
+// Measured, 512 channels x 2^20 samples, 131072 taps: 512 partitions of 256 samples 64.2 ms, error 4.4e-7; 64 of 2048
+// samples 10.4 ms (transforms 3.4, products 7.1), 2.9e-7; 32 of 4096 samples 8.7 ms (4.2, 4.3), 2.7e-7.
 static int whole_block(int block, int64_t taps) {
     int b = block;
     while (b < kWholeBlock && 2 * (int64_t)b * kWholePartitions <= taps) b *= 2;
