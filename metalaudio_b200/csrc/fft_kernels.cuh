@@ -1030,7 +1030,7 @@ inline bool istft_fast_ok(const C2RParams& p) {
             return false;
         if (p.n_partials > 1 || p.hop <= 0 || p.hop % (2 * T) != 0) return false;
         const int h = p.hop / (2 * T);
-        if (h > R || R % h != 0) return false;
+        if (h > R) return false;
         if (istft_plain<M>(p)) return true;
         if ((reinterpret_cast<uintptr_t>(p.out) & 7) != 0 || (p.out_signal_stride & 1) != 0) return false;
         return true;
@@ -1120,7 +1120,7 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
     int64_t G1 = G0 + per;
     if (G1 > total) G1 = total;
     if (G0 >= G1) return;  // uniform across the CTA
-    const int reach = R / h - 1;
+    const int reach = (R + h - 1) / h - 1;  // h need not divide R in the shared-memory ring
     int64_t s = G0 / F;
     int64_t f = G0 - s * F;
     int64_t lead = f < reach ? f : reach;

@@ -54,13 +54,13 @@ static void launch_maybe_dependent(K kernel, int grid, int threads, size_t smem,
 }
 
 // Kernels of several frames per CTA with a fixed layout but no staging fit five CTAs of 128 threads on an SM.
-template <int M, int LAYOUT>
+template <int M, bool ALIGNED, int LAYOUT>
 constexpr int r2c_ctas() {
-    return CtaShape<M>::FPC > 1 && LAYOUT >= 0 && !plan_pairable<M>() ? 5 : 512 / CtaShape<M>::THREADS;
+    return CtaShape<M>::FPC > 1 && LAYOUT >= 0 && !(ALIGNED && plan_pairable<M>()) ? 5 : 512 / CtaShape<M>::THREADS;
 }
 
 template <int M, bool ALIGNED, int LAYOUT, int MAGK, bool HALF>
-__global__ void __launch_bounds__(CtaShape<M>::THREADS, r2c_ctas<M, LAYOUT>()) r2c_kernel(const R2CParams p) {
+__global__ void __launch_bounds__(CtaShape<M>::THREADS, r2c_ctas<M, ALIGNED, LAYOUT>()) r2c_kernel(const R2CParams p) {
     DevCta cta;
     if (p.dependent_launch) dependents_launch();
     r2c_body<M, ALIGNED, LAYOUT, MAGK, DevCta, HALF>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
@@ -145,10 +145,15 @@ static ma_status launch_r2c_variant(ma_fft_plan* plan, const R2CParams& p, bool 
         if (!aligned && magk == -1 && p.layout == LAYOUT_HALF_PACKED && p.frame_valid == M && p.window == nullptr)
             return launch_r2c_t<M, true, LAYOUT_HALF_PACKED, -1, true>(plan, p);
     }
-    if constexpr (!plan_pairable<M>() && M >= 64) {
-        if (p.layout == LAYOUT_HALF_INTERLEAVED && magk == -1)
-            return aligned ? launch_r2c_t<M, true, LAYOUT_HALF_INTERLEAVED, -1>(plan, p)
-                           : launch_r2c_t<M, false, LAYOUT_HALF_INTERLEAVED, -1>(plan, p);
+    if constexpr (M >= 64) {
+        if (p.layout == LAYOUT_HALF_INTERLEAVED && magk != -2 && !aligned)
+            return magk == 0 ? launch_r2c_t<M, false, LAYOUT_HALF_INTERLEAVED, 0>(plan, p)
+                             : launch_r2c_t<M, false, LAYOUT_HALF_INTERLEAVED, -1>(plan, p);
+    }
+    if constexpr (M >= 64 && !plan_pairable<M>()) {
+        if (p.layout == LAYOUT_HALF_INTERLEAVED && magk != -2)
+            return magk == 0 ? launch_r2c_t<M, true, LAYOUT_HALF_INTERLEAVED, 0>(plan, p)
+                             : launch_r2c_t<M, true, LAYOUT_HALF_INTERLEAVED, -1>(plan, p);
     }
     return aligned ? launch_r2c_t<M, true, -1, -2>(plan, p) : launch_r2c_t<M, false, -1, -2>(plan, p);
 }
@@ -254,7 +259,10 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     const bool fast = istft_fast_ok<M>(p);
     if constexpr (CtaShape<M>::FPC >= kRowsFromSlots) {
         const size_t rows_smem = istft_rows_smem<M>(p.hop);
-        if (!fast && rows_smem <= kRowsSmemLimit) {
+        // The fast kernel's CTA is one frame's threads: less than a warp below 1024 points (256 points, hop 64: STFT and
+        // iSTFT of 256 x 300000 samples 1800 us with it, 1423 us with the rows).  The plain overlap-add of
+        // convolution blocks, which stages packed rows, is the faster one at any length.
+        if ((!fast || (T < 32 && !istft_plain<M>(p))) && rows_smem <= kRowsSmemLimit) {
             return p.layout == LAYOUT_HALF_INTERLEAVED
                        ? launch_istft_rows<M, LAYOUT_HALF_INTERLEAVED>(plan, p, rows_smem, &plan->rows_occ[0])
                        : launch_istft_rows<M, -1>(plan, p, rows_smem, &plan->rows_occ[1]);
@@ -262,21 +270,25 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     }
     const int ov = fast ? (2 * M) / p.hop : 0;
     // 0: general kernel; 1: fast, overlap count read at run time; 2: fast with the overlap count 4
-    // fixed at compile time (register ring); 3: the convolution's block overlap-add
-    const int kind = !fast ? 0 : istft_plain<M>(p) ? 3 : (ov == 4 ? 2 : 1);
-    const size_t smem = kind == 3 ? (size_t)IstftFastShape<M, 2, true>::SMEM_BYTES
+    // fixed at compile time (register ring); 3: the convolution's block overlap-add; 4: overlap count 2
+    const int kind = !fast ? 0 : istft_plain<M>(p) ? 3 : ov == 2 && 2 * p.hop == 2 * M && p.layout == LAYOUT_HALF_INTERLEAVED ? 4
+                   : (ov == 4 && 4 * p.hop == 2 * M) ? 2 : 1;
+    const size_t smem = kind == 4 ? (size_t)IstftFastShape<M, 2>::SMEM_BYTES
+                      : kind == 3 ? (size_t)IstftFastShape<M, 2, true>::SMEM_BYTES
                       : kind == 2 ? (size_t)IstftFastShape<M, 4>::SMEM_BYTES
                       : kind == 1 ? (size_t)IstftFastShape<M, 0>::SMEM_BYTES
                                   : 2 * smem_elems_per_fft<M, 1>() * sizeof(float2) + 2 * M * sizeof(float);
-    static int per_sm[4][64] = {{0}, {0}, {0}, {0}};
+    static int per_sm[5][64] = {{0}, {0}, {0}, {0}, {0}};
     ma_context* ctx = plan->ctx;
     int& occ = per_sm[kind][ctx->device & 63];
-    const int variant = !fast || kind == 3 ? 0
+    const int variant = !fast || kind >= 3 ? 0
                               : (p.layout == LAYOUT_HALF_INTERLEAVED ? 1 : (p.layout == LAYOUT_HALF_PACKED ? 3 : 5)) +
-                                    (ov == 4 ? 1 : 0);
+                                    (kind == 2 ? 1 : 0);
     if (occ == 0) {  // the layout variants of a kind share its footprint; raise every one's shared-memory limit
         int dummy;
-        if (kind == 3) {
+        if (kind == 4) {
+            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 2>, T, smem, &occ));
+        } else if (kind == 3) {
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true>, T, smem, &occ));
         } else if (kind == 2) {
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 4>, T, smem, &occ));
@@ -314,6 +326,10 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     if (grid < 1) return MA_OK;
     if (kind == 3) {
         istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true><<<grid, T, smem, ctx->stream>>>(p);
+        return after_launch(ctx);
+    }
+    if (kind == 4) {
+        istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 2><<<grid, T, smem, ctx->stream>>>(p);
         return after_launch(ctx);
     }
     switch (variant) {
