@@ -480,7 +480,7 @@ static size_t biquad_smem(int sections, int per) {
 }
 
 // Chunks per channel that fill the device once: two CTAs of 256 threads share an SM.
-constexpr int kBqSplitFrom = 3;
+constexpr int kBqSplitFrom = 4;
 static int split_max_chunks(const ma_biquad* bq) {
     if (bq->sections > kBqSplitSections) return 1;
     const int n = 2 * bq->ctx->sm_count / bq->channels;
