@@ -3,6 +3,7 @@
 #include <chrono>
 #include <cstring>
 #include <new>
+#include <system_error>
 #include <thread>
 
 #include "bulk_copy.cuh"
@@ -61,6 +62,79 @@ bool is_pinned(const void* p) {
     return a.type == cudaMemoryTypeHost;
 }
 
+// Pageable arrays cross the staging buffer in pieces.  A piece's memcpy (first touch of fresh pages above all)
+// takes several times its transfer, so arrays of 2 MiB and more are copied by up to four threads: each
+// takes every fourth piece, and transfers run while other pieces are copied.  The threads end with the call.
+constexpr size_t kThreadedCopyFrom = (size_t)2 << 20;
+static_assert(kCopyPieces % kCopyThreads == 0, "pieces are dealt out evenly");
+
+static int copy_threads() {
+    const unsigned n = std::thread::hardware_concurrency();
+    return n >= (unsigned)kCopyThreads ? kCopyThreads : 1;
+}
+
+// work(0 .. kCopyThreads-1), one of them on the calling thread; without threads to be had all of them there.
+template <class F>
+static void on_copy_threads(const F& work) {
+    std::thread pool[kCopyThreads];
+    for (int i = 1; i < kCopyThreads; ++i) {
+        try {
+            pool[i] = std::thread(work, i);
+        } catch (const std::system_error&) {
+            work(i);
+        }
+    }
+    work(0);
+    for (int i = 1; i < kCopyThreads; ++i)
+        if (pool[i].joinable()) pool[i].join();
+}
+
+// One filling of the staging buffer, host -> device (to_device) or back, in kCopyPieces pieces.
+static cudaError_t threaded_copy(ma_context* ctx, char* dptr, char* host, size_t bytes, bool to_device) {
+    const size_t piece = ((bytes + kCopyPieces - 1) / kCopyPieces + 4095) & ~(size_t)4095;
+    char* stage = (char*)ctx->pinned;
+    std::atomic<int> failed{(int)cudaSuccess};
+    auto size_of = [&](int k) { return k * piece >= bytes ? (size_t)0 : bytes - k * piece < piece ? bytes - k * piece : piece; };
+    if (!to_device) {
+        for (int k = 0; k < kCopyPieces && size_of(k) > 0; ++k) {
+            cudaError_t e = cudaMemcpyAsync(stage + k * piece, dptr + k * piece, size_of(k), cudaMemcpyDeviceToHost, ctx->stream);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_piece[k], ctx->stream);
+            if (e != cudaSuccess) {
+                (void)cudaStreamSynchronize(ctx->stream);
+                return e;
+            }
+        }
+    }
+    on_copy_threads([&](int i) {
+        cudaError_t e = i == 0 ? cudaSuccess : cudaSetDevice(ctx->device);
+        for (int k = i; k < kCopyPieces && size_of(k) > 0 && e == cudaSuccess; k += kCopyThreads) {
+            if (to_device) {
+                std::memcpy(stage + k * piece, host + k * piece, size_of(k));
+                e = cudaMemcpyAsync(dptr + k * piece, stage + k * piece, size_of(k), cudaMemcpyHostToDevice, ctx->stream);
+            } else {
+                e = cudaEventSynchronize(ctx->ev_piece[k]);
+                if (e == cudaSuccess) std::memcpy(host + k * piece, stage + k * piece, size_of(k));
+            }
+        }
+        if (e != cudaSuccess) failed.store((int)e);
+    });
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    return failed.load() != (int)cudaSuccess ? (cudaError_t)failed.load() : e;
+}
+
+static ma_status threaded_copy_all(ma_context* ctx, char* dptr, char* host, size_t bytes, bool to_device) {
+    const size_t most = (ctx->pinned_bytes / kCopyPieces & ~(size_t)4095) * kCopyPieces;
+    for (size_t off = 0; off < bytes; off += most) {
+        const size_t n = bytes - off < most ? bytes - off : most;
+        MA_CUDA(threaded_copy(ctx, dptr + off, host + off, n, to_device));
+    }
+    return MA_OK;
+}
+
+static bool copy_threaded(const ma_context* ctx, size_t bytes) {
+    return bytes >= kThreadedCopyFrom && ctx->pinned_bytes >= kThreadedCopyFrom && copy_threads() > 1;
+}
+
 ma_status copy_h2d(ma_context* ctx, void* dptr, const void* host, size_t bytes) {
     if (bytes == 0) return MA_OK;
     if (is_pinned(host)) {
@@ -68,6 +142,8 @@ ma_status copy_h2d(ma_context* ctx, void* dptr, const void* host, size_t bytes) 
         MA_CUDA(cudaStreamSynchronize(ctx->stream));
         return MA_OK;
     }
+    if (copy_threaded(ctx, bytes))
+        return threaded_copy_all(ctx, (char*)dptr, (char*)const_cast<void*>(host), bytes, true);
     const size_t half = ctx->pinned_bytes / 2;
     size_t off = 0;
     int h = 0;
@@ -92,6 +168,7 @@ ma_status copy_d2h(ma_context* ctx, void* host, const void* dptr, size_t bytes) 
         MA_CUDA(cudaStreamSynchronize(ctx->stream));
         return MA_OK;
     }
+    if (copy_threaded(ctx, bytes)) return threaded_copy_all(ctx, (char*)const_cast<void*>(dptr), (char*)host, bytes, false);
     const size_t half = ctx->pinned_bytes / 2;
     size_t off = 0, prev_off = 0, prev_n = 0;
     int h = 0;
@@ -118,6 +195,32 @@ ma_status copy_d2h(ma_context* ctx, void* host, const void* dptr, size_t bytes) 
         }
     }
     return MA_OK;
+}
+
+ma_status SmallCall::open(ma_context* context) {
+    ctx = context;
+    if (ctx->fault_site == MA_FAULT_ALLOC) return injected(ctx);
+    dev = ctx->small;
+    return MA_OK;
+}
+
+ma_status SmallCall::send() {
+    char* stage = (char*)ctx->pinned;
+    for (int i = 0; i < n_in; ++i) std::memcpy(stage + in[i].offset, in[i].host_in, in[i].bytes);
+    MA_CUDA(cudaMemcpyAsync(dev, stage, in_bytes, cudaMemcpyHostToDevice, ctx->stream));
+    return MA_OK;
+}
+
+ma_status SmallCall::receive() {
+    char* stage = (char*)ctx->pinned + in_bytes;
+    MA_CUDA(cudaMemcpyAsync(stage, dev + in_bytes, out_bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    MA_CUDA(cudaStreamSynchronize(ctx->stream));
+    for (int i = 0; i < n_out; ++i) std::memcpy(out[i].host_out, stage + out[i].offset, out[i].bytes);
+    return MA_OK;
+}
+
+void SmallCall::close(ma_status st) {
+    if (st != MA_OK) (void)cudaStreamSynchronize(ctx->stream);  // nothing may still use the staging buffer
 }
 
 ma_status workspace_lanes(ma_context* ctx, size_t min_lane_bytes, char** lane0, char** lane1, size_t* lane_bytes) {
@@ -242,9 +345,12 @@ ma_status ma_context_create(int32_t device_index, size_t pinned_bytes, ma_contex
     }
     for (int i = 0; i < 2 && e == cudaSuccess; ++i)
         e = cudaEventCreateWithFlags(&ctx->ev_half[i], cudaEventDisableTiming);
+    for (int i = 0; i < kCopyPieces && e == cudaSuccess; ++i)
+        e = cudaEventCreateWithFlags(&ctx->ev_piece[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev_begin);
     if (e == cudaSuccess) e = cudaEventCreate(&ctx->ev_end);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->ev_sync, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaMalloc((void**)&ctx->small, SmallCall::kDeviceBytes);
     if (e == cudaSuccess) e = cudaMalloc((void**)&ctx->d_error_flag, sizeof(int32_t));
     if (e == cudaSuccess) e = cudaMemsetAsync(ctx->d_error_flag, 0, sizeof(int32_t), ctx->stream);  // ordered before every kernel of the context
     if (e == cudaSuccess) e = cudaHostAlloc((void**)&ctx->h_error_flag, sizeof(int32_t), cudaHostAllocDefault);
@@ -273,10 +379,13 @@ ma_status ma_context_destroy(ma_context* ctx) {
     if (ctx->stream) (void)cudaStreamSynchronize(ctx->stream);
     for (int i = 0; i < 2; ++i)
         if (ctx->ev_half[i]) (void)cudaEventDestroy(ctx->ev_half[i]);
+    for (int i = 0; i < kCopyPieces; ++i)
+        if (ctx->ev_piece[i]) (void)cudaEventDestroy(ctx->ev_piece[i]);
     if (ctx->ev_begin) (void)cudaEventDestroy(ctx->ev_begin);
     if (ctx->ev_end) (void)cudaEventDestroy(ctx->ev_end);
     if (ctx->ev_sync) (void)cudaEventDestroy(ctx->ev_sync);
     if (ctx->pinned) (void)cudaFreeHost(ctx->pinned);
+    if (ctx->small) (void)cudaFree(ctx->small);
     if (ctx->d_error_flag) (void)cudaFree(ctx->d_error_flag);
     if (ctx->h_error_flag) (void)cudaFreeHost(ctx->h_error_flag);
     for (int i = 0; i < 2; ++i) {

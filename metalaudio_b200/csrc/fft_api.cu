@@ -328,6 +328,19 @@ ma_status ma_fft_forward_host(ma_fft_plan* plan, const float* in, float* out_a, 
         }
         return pp.finish();
     }
+    if (SmallCall::fits(ctx, in_b_ + a_b + b_b + m_b)) {
+        SmallCall call;
+        const int i_in = call.add_in(in, in_b_), o_a = call.add_out(out_a, a_b), o_b = b_b ? call.add_out(out_b, b_b) : -1,
+                  o_m = m_b ? call.add_out(mag, m_b) : -1;
+        MA_TRY(call.open(ctx));
+        ma_status st = call.send();
+        if (st == MA_OK)
+            st = ma_fft_forward_dev(plan, call.in_ptr(i_in), call.out_ptr(o_a), call.out_ptr(o_b), call.out_ptr(o_m), mag_kind,
+                                    db_reference, batch, layout);
+        if (st == MA_OK) st = call.receive();
+        call.close(st);
+        return st;
+    }
     float *d_in = nullptr, *d_a = nullptr, *d_b = nullptr, *d_m = nullptr;
     ma_status st = temp_alloc(ctx, in_b_, (void**)&d_in);
     if (st == MA_OK) st = temp_alloc(ctx, a_b, (void**)&d_a);
@@ -383,6 +396,17 @@ ma_status ma_fft_inverse_host(ma_fft_plan* plan, const float* in_a, const float*
         }
         return pp.finish();
     }
+    if (SmallCall::fits(ctx, a_b + b_b + o_b)) {
+        SmallCall call;
+        const int i_a = call.add_in(in_a, a_b), i_b = b_b ? call.add_in(in_b, b_b) : -1, o_o = call.add_out(out, o_b);
+        MA_TRY(call.open(ctx));
+        ma_status st = call.send();
+        if (st == MA_OK)
+            st = ma_fft_inverse_dev(plan, call.in_ptr(i_a), i_b < 0 ? nullptr : call.in_ptr(i_b), call.out_ptr(o_o), batch, layout);
+        if (st == MA_OK) st = call.receive();
+        call.close(st);
+        return st;
+    }
     float *d_a = nullptr, *d_b = nullptr, *d_o = nullptr;
     ma_status st = temp_alloc(ctx, a_b, (void**)&d_a);
     if (st == MA_OK && b_b) st = temp_alloc(ctx, b_b, (void**)&d_b);
@@ -410,6 +434,18 @@ ma_status ma_fft_magnitude_host(ma_fft_plan* plan, const float* re, const float*
     const size_t row = (size_t)plan->n * sizeof(float);
     const size_t in_bytes = batch == 1 ? (size_t)kh * sizeof(float) : (size_t)batch * row;
     const size_t o_b = (size_t)batch * kh * sizeof(float);
+    if (SmallCall::fits(ctx, 2 * (size_t)batch * row + o_b)) {
+        SmallCall call;
+        const int i_re = call.add_in(re, in_bytes, (size_t)batch * row), i_im = call.add_in(im, in_bytes, (size_t)batch * row),
+                  o_o = call.add_out(out, o_b);
+        MA_TRY(call.open(ctx));
+        ma_status st = call.send();
+        if (st == MA_OK)
+            st = ma_fft_magnitude_dev(plan, call.in_ptr(i_re), call.in_ptr(i_im), call.out_ptr(o_o), batch, kind, db_reference);
+        if (st == MA_OK) st = call.receive();
+        call.close(st);
+        return st;
+    }
     float *d_re = nullptr, *d_im = nullptr, *d_o = nullptr;
     ma_status st = temp_alloc(ctx, (size_t)batch * row, (void**)&d_re);
     if (st == MA_OK) st = temp_alloc(ctx, (size_t)batch * row, (void**)&d_im);

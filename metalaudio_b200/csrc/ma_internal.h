@@ -8,6 +8,7 @@
 #include "../../include/metalaudio_cuda.h"
 
 constexpr int kAuxStreams = 3;
+constexpr int kCopyPieces = 16, kCopyThreads = 4;  // threaded copies of pageable arrays (context.cu)
 
 struct ma_context {
     int device = 0;
@@ -28,12 +29,14 @@ struct ma_context {
     void* pinned = nullptr;       // staging buffer, used as two halves
     size_t pinned_bytes = 0;
     cudaEvent_t ev_half[2] = {nullptr, nullptr};
+    cudaEvent_t ev_piece[kCopyPieces] = {};
     cudaEvent_t ev_begin = nullptr, ev_end = nullptr, ev_sync = nullptr;
     bool timing_open = false;
     bool lost = false;
     int fault_site = -1;          // host-side fault injection: next call reaching the site fails
     int fault_error = 0;
     char name[256] = {0};
+    char* small = nullptr;            // device side of SmallCall, SmallCall::kDeviceBytes
     int32_t* d_error_flag = nullptr;  // set by a kernel whose bounded wait ran out
     int32_t* h_error_flag = nullptr;  // pinned mirror read at synchronisation
     // Output rows of the latest convolution streaming step on this context (any object): the next
@@ -69,6 +72,43 @@ bool is_pinned(const void* p);
 // Makes sure the context's two workspace lanes hold at least `min_lane_bytes` each (grow-only; a
 // growth waits for all queued work first).  Returns the lanes.
 ma_status workspace_lanes(ma_context* ctx, size_t min_lane_bytes, char** lane0, char** lane1, size_t* lane_bytes);
+
+// A *_host call on a few arrays of some kilobytes (one analysis frame): its inputs go to the device as one
+// transfer through the staging buffer and its results come back as one, so the call waits once instead of
+// after every array.  add_* lay the arrays out; then open, send, the kernels on in_ptr / out_ptr,
+// receive, and close in any case.  Arrays may be pageable or page-locked.
+struct SmallCall {
+    struct Part {
+        const void* host_in;
+        void* host_out;
+        size_t bytes, offset;
+    };
+    static constexpr size_t kMostBytes = (size_t)256 << 10, kDeviceBytes = kMostBytes + 8 * 256;
+    ma_context* ctx = nullptr;
+    char* dev = nullptr;
+    size_t in_bytes = 0, out_bytes = 0;
+    int n_in = 0, n_out = 0;
+    Part in[2], out[3];
+
+    static bool fits(const ma_context* c, size_t bytes) { return bytes <= kMostBytes && kDeviceBytes <= c->pinned_bytes; }
+    // `span`: device bytes the kernels may address, at least the bytes copied
+    int add_in(const void* host, size_t bytes, size_t span = 0) {
+        in[n_in] = {host, nullptr, bytes, in_bytes};
+        in_bytes += ((span > bytes ? span : bytes) + 255) & ~(size_t)255;
+        return n_in++;
+    }
+    int add_out(void* host, size_t bytes) {
+        out[n_out] = {nullptr, host, bytes, out_bytes};
+        out_bytes += (bytes + 255) & ~(size_t)255;
+        return n_out++;
+    }
+    float* in_ptr(int i) const { return reinterpret_cast<float*>(dev + in[i].offset); }
+    float* out_ptr(int i) const { return i < 0 ? nullptr : reinterpret_cast<float*>(dev + in_bytes + out[i].offset); }
+    ma_status open(ma_context* context);
+    ma_status send();
+    ma_status receive();
+    void close(ma_status st);
+};
 
 // Stream-ordered temporary device memory for the *_host entry points.
 ma_status temp_alloc(ma_context* ctx, size_t bytes, void** dptr);
