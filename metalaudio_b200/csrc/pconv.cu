@@ -238,8 +238,9 @@ __global__ void __launch_bounds__(kMacThreads) pconv_mac_kernel(const MacParams 
 // rows in a ring of 128 rows (each row enters once per CTA), the partition rows double-buffered.
 // That leaves about 0.25 byte of L2 traffic per complex multiply-accumulate and makes the FMA
 // pipe the limiter.  One barrier per chunk (1024 FMAs per thread apart).
-// A complex product is two packed two-wide multiply-adds, on the window row and on its swapped copy (64 partitions
-// of 2048 bins, 512 channels x 576 blocks: 7.50 -> 7.13 ms against four scalar ones).
+// A complex product is two packed two-wide multiply-adds into two component-wise sums: no operand has to be
+// swapped or negated (32 partitions of 4096 bins, 512 channels x 288 blocks: 4.33 -> 4.0 ms against sums
+// of complex products, for which the swapped rows were rebuilt at every use).
 // TWO_LEVEL: every kFlushChunks chunks the running sums are added into a second set of
 // accumulators and cleared, so no float32 sum runs over more than TT*kFlushChunks partitions
 // (blocked summation: the rounding error of thousands of partitions grows with the block
@@ -289,14 +290,16 @@ __global__ void __launch_bounds__(128) pconv_mac_tiled_kernel(const MacParams q,
     __pipeline_wait_prior(0);
     __syncthreads();
 
-    float2 acc[TT], xw[TT], xs_[TT];  // window rows as (re, im) and as (im, re)
+    // x*h as two component-wise sums, ar = sum (xr, xi) * hr and ai = sum (xr, xi) * hi; re = ar.x - ai.y and
+    // im = ar.y + ai.x at the end.  Packed operands are used as they lie in the window.
+    float2 ar[TT], ai[TT], xw[TT];
     float2 acc2[TWO_LEVEL ? TT : 1];
 #pragma unroll
     for (int i = 0; i < TT; ++i) {
-        acc[i] = make_float2(0.f, 0.f);
+        ar[i] = make_float2(0.f, 0.f);
+        ai[i] = make_float2(0.f, 0.f);
         if constexpr (TWO_LEVEL) acc2[i] = make_float2(0.f, 0.f);
         xw[i] = xs[(base + i) & (RING - 1)][lane];
-        xs_[i] = make_float2(xw[i].y, xw[i].x);
     }
     int buf = 0;
     int since_flush = 0;
@@ -315,18 +318,14 @@ __global__ void __launch_bounds__(128) pconv_mac_tiled_kernel(const MacParams q,
                 const int p = p0 + j;
                 if (FULL || p < P) {
                     // slot (i - j) mod TT holds timeline row base + i - p; the row base - p enters at i = 0
-                    if (j > 0 || p0 > 0) {
-                        const float2 x = xs[(base - p) & (RING - 1)][lane];
-                        xw[(TT - j) % TT] = x;
-                        xs_[(TT - j) % TT] = make_float2(x.y, x.x);
-                    }
+                    if (j > 0 || p0 > 0) xw[(TT - j) % TT] = xs[(base - p) & (RING - 1)][lane];
                     const float2 h = hrow[j * 32];
-                    const float ha = dc ? 0.f : h.y;   // bin 0 carries (DC, Nyquist): component-wise product
-                    const float2 h1 = make_float2(h.x, dc ? h.y : h.x), h2 = make_float2(-ha, ha);
+                    const float hi = dc ? 0.f : h.y;   // bin 0 carries (DC, Nyquist): component-wise product
+                    const float2 hr2 = make_float2(h.x, dc ? h.y : h.x), hi2 = make_float2(hi, hi);
 #pragma unroll
                     for (int i = 0; i < TT; ++i) {
-                        acc[i] = pfma(xw[(i - j + TT) % TT], h1, acc[i]);
-                        acc[i] = pfma(xs_[(i - j + TT) % TT], h2, acc[i]);
+                        ar[i] = pfma(xw[(i - j + TT) % TT], hr2, ar[i]);
+                        ai[i] = pfma(xw[(i - j + TT) % TT], hi2, ai[i]);
                     }
                 }
             }
@@ -338,9 +337,10 @@ __global__ void __launch_bounds__(128) pconv_mac_tiled_kernel(const MacParams q,
                 since_flush = 0;
 #pragma unroll
                 for (int i = 0; i < TT; ++i) {
-                    acc2[i].x += acc[i].x;
-                    acc2[i].y += acc[i].y;
-                    acc[i] = make_float2(0.f, 0.f);
+                    acc2[i].x += ar[i].x - ai[i].y;
+                    acc2[i].y += ar[i].y + ai[i].x;
+                    ar[i] = make_float2(0.f, 0.f);
+                    ai[i] = make_float2(0.f, 0.f);
                 }
             }
         }
@@ -348,18 +348,15 @@ __global__ void __launch_bounds__(128) pconv_mac_tiled_kernel(const MacParams q,
         __syncthreads();
         buf ^= 1;
     }
-    if constexpr (TWO_LEVEL) {
-#pragma unroll
-        for (int i = 0; i < TT; ++i) {
-            acc[i].x += acc2[i].x;
-            acc[i].y += acc2[i].y;
-        }
-    }
     const int t0 = t0_cta + warp * TT;
     float2* o = q.out + (int64_t)c * q.out_chan_stride + (int64_t)t0 * q.out_t_stride + bt * 32 + lane;
 #pragma unroll
     for (int i = 0; i < TT; ++i)
-        if (t0 + i < t_total) o[(int64_t)i * q.out_t_stride] = acc[i];
+        if (t0 + i < t_total) {
+            float2 y = make_float2(ar[i].x - ai[i].y, ar[i].y + ai[i].x);
+            if constexpr (TWO_LEVEL) y = make_float2(y.x + acc2[i].x, y.y + acc2[i].y);
+            o[(int64_t)i * q.out_t_stride] = y;
+        }
 }
 
 constexpr int kTwoLevelFrom = 2048;
