@@ -43,11 +43,12 @@ constexpr int kBqMaxSections = 32;
 //   [8..135]   A^(PER*l) row-major 2x2, l < 32 (PER: samples per thread)
 //   [136..139] A^(PER*32)
 //   [140..171] A^(PER*32*w), w < 8: a warp's worth of samples, w times over
+//   [172..235] first row of A^j, j < 32: what a unit state in front of a thread's block adds to output j
 // Time splits (few channels): cascades of up to kBqSplitSections sections; a ladder of kBqLadder matrices per
 // coefficient set, entry j the zero-input transition of the whole cascade (2S x 2S, row-major, state
 // order z1 z2 of section 0, z1 z2 of section 1, ...) over 2^j tiles.
 constexpr int kBqSplitSections = 8, kBqLadder = 9, kBqMaxChunks = 64;
-constexpr int kBqCoef = 0, kBqPl = 8, kBqPw = 136, kBqPx = 140, kBqTable = 172;
+constexpr int kBqCoef = 0, kBqPl = 8, kBqPw = 136, kBqPx = 140, kBqPy = 172, kBqTable = 236;
 
 struct BiquadLaunch {
     const float* in;
@@ -245,15 +246,22 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
             // one dependent multiply-add per sample instead of two (the output is off the chain).
             // In double precision the rearrangement changes nothing at float32 output level.
             const double b0 = T[0], a1 = T[3], a2 = T[4], c1 = T[5], c2 = T[6];
-            // ---- zero-state pass over this thread's samples: only its end state is kept
+            // ---- zero-state pass over this thread's samples: its end state and, where the samples stay in
+            // double precision, its outputs
             double z1 = 0.0, z2 = 0.0;
+            const bool add_response = DBL && !(ends_signal && last_tile) && !(MODE == BQ_ENDS && s == p.n_sections - 1);
+            auto zero_pass = [&](auto keep) {
 #pragma unroll
-            for (int j = 0; j < kBqPer; ++j) {
-                const double xv = (double)x[j];
-                const double z1n = fma(-a1, z1, fma(c1, xv, z2));
-                z2 = fma(-a2, z1, c2 * xv);
-                z1 = z1n;
-            }
+                for (int j = 0; j < kBqPer; ++j) {
+                    const double xv = (double)x[j];
+                    if (decltype(keep)::value) x[j] = (X)fma(b0, xv, z1);
+                    const double z1n = fma(-a1, z1, fma(c1, xv, z2));
+                    z2 = fma(-a2, z1, c2 * xv);
+                    z1 = z1n;
+                }
+            };
+            if (add_response) zero_pass(std::true_type{});
+            else zero_pass(std::false_type{});
             // ---- inclusive scan of the end states across the warp: E_l = P*E_{l-1} + e_l, P = A^32
             double2 e = make_double2(z1, z2);
 #pragma unroll
@@ -315,6 +323,25 @@ __global__ void __launch_bounds__(kBqThreads, 2) biquad_kernel(const BiquadLaunc
             double2 prev = make_double2(__shfl_up_sync(0xffffffffu, e.x, 1), __shfl_up_sync(0xffffffffu, e.y, 1));
             if (lane == 0) prev = make_double2(0.0, 0.0);
             const double2 pc = mat_vec(T + kBqPl + 4 * lane, c);
+            if (add_response) {
+                // the recurrence is linear: the outputs from the true state are those from the zero state plus
+                // the state's own response, two independent multiply-adds a sample instead of five in a chain
+                // (24 channels x 480000 samples, 4 sections 133 -> 130 us; 200 x 300000, 8 sections 876 -> 855 us)
+                const double2* resp = reinterpret_cast<const double2*>(T + kBqPy);
+                const double s1 = prev.x + pc.x, s2 = prev.y + pc.y;
+#pragma unroll
+                for (int j = 0; j < kBqPer; ++j) {
+                    const double2 g = resp[j];
+                    x[j] = (X)fma(g.x, s1, fma(g.y, s2, (double)x[j]));
+                }
+                if (tid == kBqThreads - 1) {
+                    const double2 m = mat_vec(T + kBqPw, c);
+                    const double2 z = make_double2(e.x + m.x, e.y + m.y);
+                    if (!last_tile) carry_out[s] = z;
+                    else if (MODE == BQ_ENDS) ends[(int64_t)(chunk + 1) * p.n_sections + s] = z;
+                }
+                continue;
+            }
             // ---- second pass from the true state in front of this thread's samples; the thread
             // that holds the signal's last sample also records the state after it
             double s1 = prev.x + pc.x, s2 = prev.y + pc.y;
@@ -410,6 +437,12 @@ static void build_table(const float* c, double* t, int per) {
         mul(P, pl, pl);
     }
     for (int i = 0; i < 4; ++i) t[kBqPw + i] = pl[i];  // A^(32*per)
+    double py[4] = {1.0, 0.0, 0.0, 1.0};
+    for (int j = 0; j < 32; ++j) {
+        t[kBqPy + 2 * j] = py[0];
+        t[kBqPy + 2 * j + 1] = py[1];
+        mul(A, py, py);
+    }
     double px[4] = {1.0, 0.0, 0.0, 1.0};
     for (int w = 0; w < kBqWarps; ++w) {
         for (int i = 0; i < 4; ++i) t[kBqPx + 4 * w + i] = px[i];
