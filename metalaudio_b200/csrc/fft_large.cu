@@ -29,6 +29,7 @@
 #include "bulk_copy.cuh"
 #include "fft_plan.h"
 #include "host_tables.h"
+#include "tensor_map.h"
 
 namespace ma {
 
@@ -756,11 +757,8 @@ static TensorMapEncodeFn tensor_map_encoder() {
     return reinterpret_cast<TensorMapEncodeFn>(cached.load(std::memory_order_acquire));
 }
 
-// Tensor map of `batch` dense [rows][row_floats] float arrays `batch_stride` floats apart, with boxes of
-// box_rows x box_floats; false when the array does not qualify (alignment, stride) or the driver cannot
-// encode it.
-static bool tile_tensor_map(const float* base, int64_t row_floats, int64_t rows, int64_t batch, int64_t batch_stride,
-                            int box_floats, int box_rows, CUtensorMap* map) {
+bool tile_tensor_map(const float* base, int64_t row_floats, int64_t rows, int64_t batch, int64_t batch_stride,
+                     int box_floats, int box_rows, CUtensorMap* map) {
     if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || (batch_stride & 3) != 0 || (row_floats & 3) != 0 ||
         batch_stride < rows * row_floats || batch > (int64_t)1 << 30)
         return false;

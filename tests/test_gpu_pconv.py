@@ -231,6 +231,23 @@ def test_whole_signal_after_steps_and_back(device, lib, block, taps):
     assert o64.rel_rms(y, np.stack([o64.convolve_full(x[i, :block], h)[:block] for i in range(channels)])) <= TOL
 
 
+@pytest.mark.parametrize("block,taps,length", [(32, 1, 32), (32, 33, 500), (32, 255, 2049), (32, 511, 1500), (4096, 65536, 5000),
+                                               (4096, 65537, 60000), (4096, 135000, 130000), (4096, 262144, 9000),
+                                               (4096, 262145, 9000)])
+def test_whole_signal_products_at_chunk_and_tile_edges(device, block, taps, length):
+    """1 to 65 partitions (64 is the last count whose rows are brought in as boxes), whole and partial chunks of
+    16, one to four warps of output blocks per CTA, one response per channel."""
+    rng = np.random.default_rng(taps)
+    channels = 3
+    h = (rng.standard_normal((2, taps)) / np.sqrt(taps)).astype(np.float32)
+    x = rng.standard_normal((channels, length)).astype(np.float32)
+    c = conv(device, block, channels=channels)
+    c.setKernel(h, channelToKernel=[1, 0, 1])
+    y = c.process(x)
+    for i, ir in enumerate([1, 0, 1]):
+        assert o64.rel_rms(y[i], o64.convolve_full(x[i], h[ir])) <= TOL
+
+
 def test_config3_scaled(device):
     """Configuration 3 at reduced channel count / length: one shared exponentially decaying
     noise IR, block 256, float64 oracle plus exact dot-product spot checks."""
