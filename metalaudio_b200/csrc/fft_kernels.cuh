@@ -873,6 +873,65 @@ MA_HD void istft_body(const C2RParams& p, Cta& cta, float2* smem) {
     }
 }
 
+// Adds up and stores the output positions [first*hop, end) counted from the start of frame fb, which sits in row
+// `base` (see istft_rows_body).  V = 2: pairs of positions, for even hops, where both are covered by the same frames.
+// With one position per thread and step this sum took as many instructions as the transform (frames of 512 points,
+// hop 160: iSTFT of 512 x 1017 frames 737 -> 577 us with pairs and one running row index).
+template <int M, int V, int THREADS>
+MA_HD void rows_emit(const C2RParams& p, const float* rows, int tid, int64_t s, int64_t fb, int base, int nb, int first, int end,
+                     int n_rows, int k_full, int r_full, bool normalise) {
+    constexpr int N = 2 * M;
+    const int hop = p.hop;
+    const int64_t F = p.frames_per_signal, start = fb * (int64_t)hop;
+    float* out = p.out + s * p.out_signal_stride + start;
+    const bool pairs = V == 2 && (reinterpret_cast<uintptr_t>(out) & 7) == 0;
+    const bool edges = start < (int64_t)(N - hop) || fb + nb == F;  // some positions lack frames on one side
+    int i = first * hop + V * tid;
+    int j = i / hop, r = i - j * hop;
+    for (; i < end; i += V * THREADS) {
+        // frames fb + j - k, k = most .. least, cover the position at offset r + k*hop
+        int most = r <= r_full ? k_full : k_full - 1;
+        if (most > fb + j) most = (int)(fb + j);
+        const int least = j >= nb ? j - (nb - 1) : 0;
+        int row = base + j - most;
+        if (row < 0) row += n_rows;
+        else if (row >= n_rows) row -= n_rows;
+        int at = row * N + r + most * hop;
+        float2 acc = make_float2(0.f, 0.f);
+        for (int k = most; k >= least; --k) {
+            if constexpr (V == 2) acc = cadd(acc, *reinterpret_cast<const float2*>(rows + at));
+            else acc.x += rows[at];
+            at += N - hop;
+            if (++row == n_rows) {
+                row = 0;
+                at -= n_rows * N;
+            }
+        }
+        if (normalise) {
+            const int64_t o = start + i;
+            // interior positions (all overlapping frames exist) share hop distinct sums
+            if (!edges || (o >= (int64_t)(N - hop) && o < F * (int64_t)hop)) {
+                acc.x *= MA_LDG(p.norm_mid_inv + r);
+                if (V == 2) acc.y *= MA_LDG(p.norm_mid_inv + r + 1);
+            } else {
+                acc.x /= window_sum_edge(p, o, N, hop, F);
+                if (V == 2 && i + 1 < end) acc.y /= window_sum_edge(p, o + 1, N, hop, F);
+            }
+        }
+        if (V == 2 && pairs && i + 1 < end) {
+            *reinterpret_cast<float2*>(out + i) = acc;
+        } else {
+            out[i] = acc.x;
+            if (V == 2 && i + 1 < end) out[i + 1] = acc.y;
+        }
+        r += V * THREADS;
+        while (r >= hop) {
+            r -= hop;
+            ++j;
+        }
+    }
+}
+
 // iSTFT of short frames (several fit a CTA) at any hop.  istft_body gives a frame to a CTA of its own, which
 // below 1024 points is less than one full warp.  Here the CTA's slots transform consecutive frames
 // side by side and leave the windowed samples in a ring of rows in shared memory; then all threads
@@ -914,7 +973,6 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
         const int64_t f0 = G - s * F;
         const int64_t f1 = f0 + (G1 - G) < F ? f0 + (G1 - G) : F;
         G += f1 - f0;
-        float* out = p.out + s * p.out_signal_stride;
         int base = 0;  // row of frame fb
         for (int64_t fb = f0 > reach ? f0 - reach : 0; fb < f1; fb += FPC) {
             const int nb = f1 - fb < FPC ? (int)(f1 - fb) : FPC;
@@ -937,34 +995,8 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
             const int64_t start = fb * (int64_t)hop;
             int end = fb + nb == F ? (nb - 1) * hop + N : nb * hop;
             if (start + end > p.out_len) end = (int)(p.out_len - start);
-            int i = first * hop + tid;
-            int j = i / hop, r = i - j * hop;
-            for (; i < end; i += S::THREADS) {
-                // frames fb + j - k, k = most .. least, cover the position at offset r + k*hop
-                int most = r <= r_full ? k_full : k_full - 1;
-                if (most > fb + j) most = (int)(fb + j);
-                const int least = j >= nb ? j - (nb - 1) : 0;
-                float acc = 0.f;
-                int row = base + j - most;
-                if (row < 0) row += n_rows;
-                else if (row >= n_rows) row -= n_rows;
-                for (int k = most; k >= least; --k) {
-                    acc += rows[row * N + r + k * hop];
-                    if (++row == n_rows) row = 0;
-                }
-                if (normalise) {
-                    const int64_t o = start + i;
-                    // interior positions (all overlapping frames exist) share hop distinct sums
-                    if (o >= (int64_t)(N - hop) && o < F * (int64_t)hop) acc *= MA_LDG(p.norm_mid_inv + r);
-                    else acc = acc / window_sum_edge(p, o, N, hop, F);
-                }
-                out[start + i] = acc;
-                r += S::THREADS;
-                while (r >= hop) {
-                    r -= hop;
-                    ++j;
-                }
-            }
+            if ((hop & 1) == 0) rows_emit<M, 2, S::THREADS>(p, rows, tid, s, fb, base, nb, first, end, n_rows, k_full, r_full, normalise);
+            else rows_emit<M, 1, S::THREADS>(p, rows, tid, s, fb, base, nb, first, end, n_rows, k_full, r_full, normalise);
             base += FPC;
             if (base >= n_rows) base -= n_rows;
             // the next batch's rows are written behind at least one barrier of its transform
