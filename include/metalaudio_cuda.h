@@ -321,7 +321,11 @@ ma_status ma_pconv_step_splits(ma_pconv* pc, int32_t set_to, int32_t* splits);
  * ma_pconv_reserve bounds len for the _dev form, which never allocates.  The _host form sends
  * groups of channels through the context's workspace lanes; with both host arrays pinned the
  * groups' copies in, convolutions and copies out overlap on three streams (see
- * ma_context_reserve_workspace). */
+ * ma_context_reserve_workspace).
+ * ma_pconv_reserve also lays the taps out in coarser blocks (up to 4096 samples, at least eight partitions of
+ * them) that whole-signal calls on a clear delay line run on: 8 more bytes per tap; without the memory the
+ * calls keep block_size.  A non-finite input sample then spoils its whole coarse block besides the reach of the
+ * response, where calls that continue a stream spoil its block of block_size samples. */
 ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len);
 ma_status ma_pconv_process_dev(ma_pconv* pc, const float* in, int64_t len, int64_t in_stride,
                                float* out, int64_t out_stride);
