@@ -83,12 +83,12 @@ __global__ void __launch_bounds__(FftPlan<M>::T, (512 / FftPlan<M>::T) > 16 ? 16
     istft_body<M, DevCta>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
 }
 
-template <int M, int LAYOUT, int OVT, bool PLAIN = false>
+template <int M, int LAYOUT, int OVT, bool PLAIN = false, bool EXACT = PLAIN>
 __global__ void __launch_bounds__(FftPlan<M>::T, (512 / FftPlan<M>::T) > 16 ? 16 : (512 / FftPlan<M>::T))
 istft_fast_kernel(const C2RParams p) {
     DevCta cta;
     if constexpr (plan_pairable<M>())
-        istft_fast_body<M, LAYOUT, OVT, DevCta, PLAIN>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
+        istft_fast_body<M, LAYOUT, OVT, DevCta, PLAIN, EXACT>(p, cta, reinterpret_cast<float2*>(ma_dyn_smem));
 }
 
 template <int M, int LAYOUT>
@@ -270,15 +270,16 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     }
     const int ov = fast ? (2 * M) / p.hop : 0;
     // 0: general kernel; 1: fast, overlap count read at run time; 2: fast with the overlap count 4
-    // fixed at compile time (register ring); 3: the convolution's block overlap-add; 4: overlap count 2
+    // fixed at compile time (register ring); 3: the convolution's block overlap-add; 4: overlap count 2;
+    // 5: a hop that does not divide the frame
     const int kind = !fast ? 0 : istft_plain<M>(p) ? 3 : ov == 2 && 2 * p.hop == 2 * M && p.layout == LAYOUT_HALF_INTERLEAVED ? 4
-                   : (ov == 4 && 4 * p.hop == 2 * M) ? 2 : 1;
+                   : (ov == 4 && 4 * p.hop == 2 * M) ? 2 : (2 * M) % p.hop != 0 ? 5 : 1;
     const size_t smem = kind == 4 ? (size_t)IstftFastShape<M, 2>::SMEM_BYTES
                       : kind == 3 ? (size_t)IstftFastShape<M, 2, true>::SMEM_BYTES
                       : kind == 2 ? (size_t)IstftFastShape<M, 4>::SMEM_BYTES
-                      : kind == 1 ? (size_t)IstftFastShape<M, 0>::SMEM_BYTES
+                      : kind == 1 || kind == 5 ? (size_t)IstftFastShape<M, 0>::SMEM_BYTES
                                   : 2 * smem_elems_per_fft<M, 1>() * sizeof(float2) + 2 * M * sizeof(float);
-    static int per_sm[5][64] = {{0}, {0}, {0}, {0}, {0}};
+    static int per_sm[6][64] = {{0}, {0}, {0}, {0}, {0}, {0}};
     ma_context* ctx = plan->ctx;
     int& occ = per_sm[kind][ctx->device & 63];
     const int variant = !fast || kind >= 3 ? 0
@@ -286,7 +287,9 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
                                     (kind == 2 ? 1 : 0);
     if (occ == 0) {  // the layout variants of a kind share its footprint; raise every one's shared-memory limit
         int dummy;
-        if (kind == 4) {
+        if (kind == 5) {
+            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0, false, true>, T, smem, &occ));
+        } else if (kind == 4) {
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 2>, T, smem, &occ));
         } else if (kind == 3) {
             MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true>, T, smem, &occ));
@@ -326,6 +329,10 @@ static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     if (grid < 1) return MA_OK;
     if (kind == 3) {
         istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true><<<grid, T, smem, ctx->stream>>>(p);
+        return after_launch(ctx);
+    }
+    if (kind == 5) {
+        istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0, false, true><<<grid, T, smem, ctx->stream>>>(p);
         return after_launch(ctx);
     }
     if (kind == 4) {

@@ -106,6 +106,7 @@ int emul_istft(int n, int hop, const float* in_a, const float* in_b, long long i
         run_grid(nblocks, FftPlan<MM>::T, smem, [&](HostCta& cta, void* sm) {                    \
             if constexpr (plan_pairable<MM>()) {                                                 \
                 if (fast && 2 * MM / hop == 4) { istft_fast_body<MM, 0, 4, HostCta>(p, cta, (float2*)sm); return; } \
+                if (fast && n % hop != 0) { istft_fast_body<MM, 0, 0, HostCta, false, true>(p, cta, (float2*)sm); return; } \
                 if (fast) { istft_fast_body<MM, 0, 0, HostCta>(p, cta, (float2*)sm); return; }   \
             }                                                                                    \
             istft_body<MM, HostCta>(p, cta, (float2*)sm);                                        \

@@ -120,6 +120,27 @@ def test_stft_istft(emul, n, hop, length, chunks, kind):
     assert o64.rel_rms(y[:, msk], yref[:, msk]) <= 1e-5
 
 
+@pytest.mark.parametrize("n,hop", [(1024, 320), (1024, 960), (2048, 640), (4096, 1280), (4096, 768), (8192, 2560)])
+def test_fast_istft_at_hops_that_do_not_divide_the_frame(emul, n, hop):
+    """The thread-private ring at 5/16, 15/16 and 3/16 of a frame: more lead-in frames than whole overlaps, slots
+    that wrap, ranges that start inside a signal."""
+    f, signals = 9, 2
+    out_len = (f - 1) * hop + n
+    rng = np.random.default_rng(n + hop)
+    w = rp.window("hamming", n)
+    x = rng.standard_normal((signals, f, n)).astype(np.float32)
+    spec = np.ascontiguousarray(np.fft.rfft(x, axis=-1).astype(np.complex64)).view(np.float32)
+    y = np.zeros((signals, out_len), np.float32)
+    assert emul.emul_istft(n, hop, fp(spec), None, f * (n // 2 + 1), n // 2 + 1, f, signals, 0, fp(w), 1e-8, fp(y), out_len,
+                           out_len, 2, 4) == 1
+    ref, ws = np.zeros((signals, out_len)), np.zeros(out_len)
+    w64 = w.astype(np.float64)
+    for k in range(f):
+        ref[:, k * hop:k * hop + n] += x[:, k] * w64
+        ws[k * hop:k * hop + n] += w64 ** 2
+    assert o64.rel_rms(y, ref / np.maximum(ws, 1e-8)) <= 1e-6
+
+
 @pytest.mark.parametrize("n", [64, 256, 1024, 2048, 4096])
 @pytest.mark.parametrize("length_off,stride_mod,cut", [(0, 0, 0), (-1, 0, 1), (3, 1, 2), (-5, 3, 7)])
 def test_convolution_block_transforms(emul, n, length_off, stride_mod, cut):
