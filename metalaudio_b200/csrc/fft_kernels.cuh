@@ -876,9 +876,9 @@ MA_HD void istft_body(const C2RParams& p, Cta& cta, float2* smem) {
 // Adds up and stores the output positions [first*hop, end) counted from the start of frame fb, which sits in row
 // `base` (see istft_rows_body).  V = 2: pairs of positions, for even hops, where both are covered by the same frames.
 // With one position per thread and step this sum took as many instructions as the transform (frames of 512 points,
-// hop 160: iSTFT of 512 x 1017 frames 737 -> 577 us with pairs and one running row index).
+// hop 160: iSTFT of 512 x 1017 frames 737 -> 610 us with pairs and one running row index).
 template <int M, int V, int THREADS>
-MA_HD void rows_emit(const C2RParams& p, const float* rows, int tid, int64_t s, int64_t fb, int base, int nb, int first, int end,
+MA_HD void rows_emit(const C2RParams& p, const float* rows, const float* window, int tid, int64_t s, int64_t fb, int base, int nb, int first, int end,
                      int n_rows, int k_full, int r_full, bool normalise) {
     constexpr int N = 2 * M;
     const int hop = p.hop;
@@ -896,11 +896,14 @@ MA_HD void rows_emit(const C2RParams& p, const float* rows, int tid, int64_t s, 
         int row = base + j - most;
         if (row < 0) row += n_rows;
         else if (row >= n_rows) row -= n_rows;
-        int at = row * N + r + most * hop;
+        int wat = r + most * hop;
+        int at = row * N + wat;
         float2 acc = make_float2(0.f, 0.f);
         for (int k = most; k >= least; --k) {
-            if constexpr (V == 2) acc = cadd(acc, *reinterpret_cast<const float2*>(rows + at));
-            else acc.x += rows[at];
+            // window and sum in one rounding, as the one-frame kernel's ring
+            if constexpr (V == 2) acc = pfma(*reinterpret_cast<const float2*>(rows + at), *reinterpret_cast<const float2*>(window + wat), acc);
+            else acc.x = fmaf(rows[at], window[wat], acc.x);
+            wat -= hop;
             at += N - hop;
             if (++row == n_rows) {
                 row = 0;
@@ -935,8 +938,8 @@ MA_HD void rows_emit(const C2RParams& p, const float* rows, int tid, int64_t s, 
 
 // iSTFT of short frames (several fit a CTA) at any hop.  istft_body gives a frame to a CTA of its own, which
 // below 1024 points is less than one full warp.  Here the CTA's slots transform consecutive frames
-// side by side and leave the windowed samples in a ring of rows in shared memory; then all threads
-// add up, per output position, the rows that cover it (in frame order, as everywhere) and store the
+// side by side and leave the samples in a ring of rows in shared memory; then all threads add up,
+// per output position, the rows that cover it times the window (in frame order, as everywhere) and store the
 // completed samples contiguously.  A CTA owns a contiguous range of the global frame list like
 // istft_fast_body and rebuilds the `reach` frames in front of it.
 // smem: exchange buffer | window times 1/N [N] floats | rows [FPC + reach][N] floats.  One exchange buffer and the
@@ -962,7 +965,7 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
     const int n_rows = FPC + reach;
     const int k_full = (N - 1) / hop, r_full = (N - 1) - k_full * hop;  // frames covering offset r: k_full + (r <= r_full)
 
-    for (int n = tid; n < M; n += S::THREADS)  // read behind the first batch's barriers
+    for (int n = tid; n < M; n += S::THREADS)  // read behind the first batch's barriers, at the sums
         wtab[n] = p.window != nullptr ? make_float2(MA_LDG(p.window + 2 * n) * scale, MA_LDG(p.window + 2 * n + 1) * scale)
                                       : make_float2(scale, scale);
     const int64_t total = p.n_signals * F;
@@ -985,10 +988,7 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
                 if (row >= n_rows) row -= n_rows;
                 float2* dst = reinterpret_cast<float2*>(rows + row * N);
 #pragma unroll
-                for (int q = 0; q < R; ++q) {
-                    const float2 w = wtab[t + q * T];
-                    dst[t + q * T] = make_float2(v[q].y * w.x, v[q].x * w.y);
-                }
+                for (int q = 0; q < R; ++q) dst[t + q * T] = make_float2(v[q].y, v[q].x);
             }
             cta.sync();
             // positions the frames of this batch complete, counted from frame fb's start
@@ -996,8 +996,8 @@ MA_HD void istft_rows_body(const C2RParams& p, Cta& cta, float2* smem) {
             const int64_t start = fb * (int64_t)hop;
             int end = fb + nb == F ? (nb - 1) * hop + N : nb * hop;
             if (start + end > p.out_len) end = (int)(p.out_len - start);
-            if ((hop & 1) == 0) rows_emit<M, 2, S::THREADS>(p, rows, tid, s, fb, base, nb, first, end, n_rows, k_full, r_full, normalise);
-            else rows_emit<M, 1, S::THREADS>(p, rows, tid, s, fb, base, nb, first, end, n_rows, k_full, r_full, normalise);
+            if ((hop & 1) == 0) rows_emit<M, 2, S::THREADS>(p, rows, reinterpret_cast<const float*>(wtab), tid, s, fb, base, nb, first, end, n_rows, k_full, r_full, normalise);
+            else rows_emit<M, 1, S::THREADS>(p, rows, reinterpret_cast<const float*>(wtab), tid, s, fb, base, nb, first, end, n_rows, k_full, r_full, normalise);
             base += FPC;
             if (base >= n_rows) base -= n_rows;
             // the next batch's rows are written behind at least one barrier of its transform
@@ -1295,12 +1295,9 @@ MA_HD void istft_fast_body(const C2RParams& p, Cta& cta, float2* smem) {
 #pragma unroll
         for (int q = 0; q < (REGRING ? 0 : R); ++q) {
             float2* slot = ring + ((q + rot) & (R - 1)) * T + t;
-            float2 acc = make_float2(v[q].y * wreg[REGRING ? 0 : q].x, v[q].x * wreg[REGRING ? 0 : q].y);
-            if (q < R - h) {  // slot already holds earlier frames
-                const float2 old = *slot;
-                acc.x += old.x;
-                acc.y += old.y;
-            }
+            const float2 w = wreg[REGRING ? 0 : q];
+            const float2 old = q < R - h ? *slot : make_float2(0.f, 0.f);  // slots that already hold earlier frames
+            const float2 acc = make_float2(fmaf(v[q].y, w.x, old.x), fmaf(v[q].x, w.y, old.y));
             if (q < h || last) {  // complete after this frame: emit
                 if (emit) {
                     const int i0 = 2 * (t + q * T);
