@@ -14,8 +14,12 @@
  *  - `_dev` entry points take device pointers, are ordered on the context's stream, do
  *    not allocate and do not synchronise.  `_host` entry points take host pointers,
  *    copy through the context (directly when the memory is pinned, e.g. from
- *    ma_host_alloc, through the context's pinned staging buffer otherwise) and return
- *    after the result is in the caller's buffer.
+ *    ma_host_alloc, through the context's pinned staging buffer otherwise; calls of the
+ *    plain transforms and magnitudes that move 256 KiB or less go through it either way, one
+ *    transfer in and one out) and return after the result is in the caller's buffer.
+ *  - objects of one context may be used from several threads, each object by one thread at a
+ *    time: `_host` calls and ma_memcpy_* that go through the context's staging buffer or
+ *    workspace wait for one another.
  *  - all data is float32; complex data is interleaved (re, im) unless a layout says
  *    otherwise; all index arithmetic is 64-bit and overflow-checked on the host.
  *  - there is no CPU fallback: without a usable CUDA device every call fails.

@@ -142,6 +142,7 @@ ma_status copy_h2d(ma_context* ctx, void* dptr, const void* host, size_t bytes) 
         MA_CUDA(cudaStreamSynchronize(ctx->stream));
         return MA_OK;
     }
+    const std::lock_guard<std::recursive_mutex> held(ctx->host_path);
     if (copy_threaded(ctx, bytes))
         return threaded_copy_all(ctx, (char*)dptr, (char*)const_cast<void*>(host), bytes, true);
     const size_t half = ctx->pinned_bytes / 2;
@@ -168,6 +169,7 @@ ma_status copy_d2h(ma_context* ctx, void* host, const void* dptr, size_t bytes) 
         MA_CUDA(cudaStreamSynchronize(ctx->stream));
         return MA_OK;
     }
+    const std::lock_guard<std::recursive_mutex> held(ctx->host_path);
     if (copy_threaded(ctx, bytes)) return threaded_copy_all(ctx, (char*)const_cast<void*>(dptr), (char*)host, bytes, false);
     const size_t half = ctx->pinned_bytes / 2;
     size_t off = 0, prev_off = 0, prev_n = 0;
@@ -199,6 +201,7 @@ ma_status copy_d2h(ma_context* ctx, void* host, const void* dptr, size_t bytes) 
 
 ma_status SmallCall::open(ma_context* context) {
     ctx = context;
+    held = std::unique_lock<std::recursive_mutex>(ctx->host_path);
     if (ctx->fault_site == MA_FAULT_ALLOC) return injected(ctx);
     dev = ctx->small;
     return MA_OK;
@@ -221,10 +224,12 @@ ma_status SmallCall::receive() {
 
 void SmallCall::close(ma_status st) {
     if (st != MA_OK) (void)cudaStreamSynchronize(ctx->stream);  // nothing may still use the staging buffer
+    held.unlock();
 }
 
 ma_status workspace_lanes(ma_context* ctx, size_t min_lane_bytes, char** lane0, char** lane1, size_t* lane_bytes) {
     constexpr size_t kDefaultLane = (size_t)256 << 20;
+    const std::lock_guard<std::recursive_mutex> held(ctx->host_path);
     if (ctx->ws == nullptr || ctx->ws_lane_bytes < min_lane_bytes) {
         if (ctx->fault_site == MA_FAULT_ALLOC) return injected(ctx);
         size_t want = ctx->ws == nullptr && min_lane_bytes < kDefaultLane ? kDefaultLane : min_lane_bytes;

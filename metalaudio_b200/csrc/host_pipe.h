@@ -20,6 +20,7 @@ struct Pipe {
     bool pinned;
     int64_t chunk;  // signals per chunk
     char* lane[2];
+    std::unique_lock<std::recursive_mutex> held;  // the lanes and their events, from pipe_open to finish
     ma_status st = MA_OK;
 
     void before_copy_in(int64_t c) {
@@ -76,6 +77,7 @@ struct Pipe {
             else if (e2 != cudaSuccess) st = cuda_fail(e2);
             else if (e3 != cudaSuccess) st = cuda_fail(e3);
         }
+        held.unlock();
         return st;
     }
     void fail(cudaError_t e) {
@@ -86,6 +88,7 @@ struct Pipe {
 // Chunk size and lanes for rows that need `row_bytes` of workspace each (sub-buffers included).
 inline ma_status pipe_open(Pipe& p, ma_context* ctx, bool pinned, int64_t rows, size_t row_bytes, size_t fixed_bytes) {
     size_t lane_bytes = 0;
+    p.held = std::unique_lock<std::recursive_mutex>(ctx->host_path);
     MA_TRY(workspace_lanes(ctx, row_bytes + fixed_bytes, &p.lane[0], &p.lane[1], &lane_bytes));
     int64_t chunk = (int64_t)((lane_bytes - fixed_bytes) / row_bytes);
     if (chunk < 1) chunk = 1;

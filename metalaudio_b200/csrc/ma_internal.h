@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 
 #include "../../include/metalaudio_cuda.h"
 
@@ -13,6 +14,11 @@ constexpr int kCopyPieces = 16, kCopyThreads = 4;  // threaded copies of pageabl
 struct ma_context {
     int device = 0;
     int sm_count = 0;
+    // What the *_host calls of a context share between host and device: the staging buffer and its events, the
+    // device block of SmallCall, the workspace lanes and their events.  A call holds the lock from the first
+    // write into any of them to the last read, so objects of one context may be called from a thread each.
+    // Recursive: a pipelined call copies pageable arrays through the staging buffer.
+    std::recursive_mutex host_path;
     cudaStream_t stream = nullptr;
     cudaStream_t copy_stream = nullptr;   // host -> device leg of the pipelined *_host calls
     cudaStream_t d2h_stream = nullptr;    // device -> host leg
@@ -86,6 +92,7 @@ struct SmallCall {
     static constexpr size_t kMostBytes = (size_t)256 << 10, kDeviceBytes = kMostBytes + 8 * 256;
     ma_context* ctx = nullptr;
     char* dev = nullptr;
+    std::unique_lock<std::recursive_mutex> held;  // from open to close
     size_t in_bytes = 0, out_bytes = 0;
     int n_in = 0, n_out = 0;
     Part in[2], out[3];

@@ -150,3 +150,114 @@ def test_plain_transforms_host_pinned_chunks(lib, small_device, n, batch):
         assert o64.rel_rms(y, xs) <= TOL
     finally:
         pin.close()
+
+
+@pytest.mark.parametrize("kind,pinned", [("frame", (True, True)), ("frame", (True, False)), ("frame", (False, False)),
+                                         ("stft", (True, True)), ("stft", (True, False)), ("stft", (False, False))])
+def test_two_threads_with_an_object_each_on_one_context(lib, small_device, kind, pinned):
+    """Two threads, each with its own FFT object and arrays on ONE context: single frames (small calls through
+    the staging buffer) and STFTs of several MiB (threaded copies, workspace lanes).  Both must get what a single
+    thread gets, bit for bit."""
+    import threading
+
+    from metalaudio_b200 import FFT, WindowType
+    from metalaudio_b200 import _lib as L
+    dev = small_device
+    assert lib.ma_context_reserve_workspace(dev.handle, 8 << 20) == 0
+    n, rounds = (2048, 300) if kind == "frame" else (1024, 8)
+    signals, length, hop = 6, 200000, 256
+    pin = Pinned(lib, dev)
+    try:
+        calls, results = [], []
+        for k in range(2):
+            f = FFT(dev, FFT.Config(size=n, windowType=WindowType.none, hopSize=hop))
+            array = pin.array if pinned[k] else lambda shape: np.zeros(shape, np.float32)
+            rng = np.random.default_rng(70 + k)
+            if kind == "frame":
+                x, re, im, back = (array((n,)) for _ in range(4))
+                mag = array((n // 2 + 1,))
+                frames = rng.standard_normal((rounds, n)).astype(np.float32)
+
+                def call(i, f=f, x=x, re=re, im=im, back=back, mag=mag, frames=frames):
+                    x[:] = frames[i]
+                    assert lib.ma_fft_forward_host(f._h, ptr(x), ptr(re), ptr(im), None, 0, 1.0, 1, L.LAYOUT_FULL_SPLIT) == 0
+                    assert lib.ma_fft_magnitude_host(f._h, ptr(re), ptr(im), ptr(mag), 1, L.MAG_MAGNITUDE, 1.0) == 0
+                    assert lib.ma_fft_inverse_host(f._h, ptr(re), ptr(im), ptr(back), 1, L.LAYOUT_FULL_SPLIT) == 0
+                    return [a.copy() for a in (re, im, mag, back)]
+            else:
+                x = array((signals, length))
+                spec = array((signals, f.frameCount(length), n // 2 + 1, 2))
+                base = rng.standard_normal(x.shape).astype(np.float32)
+
+                def call(i, f=f, x=x, spec=spec, base=base):
+                    x[:] = base * np.float32(i + 1)
+                    assert lib.ma_stft_host(f._h, ptr(x), length, length, signals, ptr(spec), None, None, 0, 1.0,
+                                            L.LAYOUT_HALF_INTERLEAVED) == 0
+                    return [spec.copy()]
+            calls.append(call)
+            results.append([call(i) for i in range(rounds)])
+        got, failed = [[], []], []
+
+        def work(k):
+            try:
+                got[k] = [calls[k](i) for i in range(rounds)]
+            except AssertionError as e:
+                failed.append(e)
+        threads = [threading.Thread(target=work, args=(k,)) for k in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join(120)
+        assert not failed
+        for k in range(2):
+            assert len(got[k]) == rounds
+            for a, b in zip(got[k], results[k]):
+                assert all(np.array_equal(p, q) for p, q in zip(a, b))
+    finally:
+        pin.close()
+
+
+@pytest.mark.parametrize("n,batch", [(2048, 12), (2048, 13), (16384, 1), (16384, 2)])
+@pytest.mark.parametrize("pinned", [True, False])
+def test_small_calls_around_their_threshold(lib, small_device, n, batch, pinned):
+    """Plain transforms just below and above the 256 KiB that go through the staging buffer as one transfer each
+    way, in place as well (the input array is the output array of the inverse)."""
+    from metalaudio_b200 import FFT, WindowType
+    from metalaudio_b200 import _lib as L
+    dev = small_device
+    f = FFT(dev, FFT.Config(size=n, windowType=WindowType.none))
+    kh = n // 2 + 1
+    pin = Pinned(lib, dev)
+    try:
+        array = pin.array if pinned else lambda shape: np.zeros(shape, np.float32)
+        x, spec, mag = array((batch, n)), array((batch, kh, 2)), array((batch, kh))
+        x[:] = np.random.default_rng(n + batch).standard_normal(x.shape)
+        keep = np.array(x)
+        assert lib.ma_fft_forward_host(f._h, ptr(x), ptr(spec), None, ptr(mag), L.MAG_MAGNITUDE, 1.0, batch,
+                                       L.LAYOUT_HALF_INTERLEAVED) == 0
+        ref = o64.rfft(keep)
+        assert o64.rel_rms(spec[..., 0] + 1j * spec[..., 1], ref) <= TOL
+        assert o64.rel_rms(mag, np.abs(ref)) <= TOL
+        assert lib.ma_fft_inverse_host(f._h, ptr(spec), None, ptr(spec), batch, L.LAYOUT_HALF_INTERLEAVED) == 0
+        assert o64.rel_rms(spec.reshape(-1)[:batch * n].reshape(batch, n), keep) <= TOL
+    finally:
+        pin.close()
+
+
+@pytest.mark.parametrize("nbytes", [(2 << 20) - 4, 2 << 20, (2 << 20) + 4, (64 << 20) - 4, (64 << 20) + 8, 130 << 20])
+def test_pageable_copies_around_the_threaded_threshold(lib, small_device, nbytes):
+    """ma_memcpy_h2d / _d2h of pageable arrays from one thread's double buffering to four threads' pieces, and across
+    several fillings of the 64 MiB staging buffer; bytes past either end stay."""
+    dev = small_device
+    count = nbytes // 4
+    x = np.random.default_rng(nbytes).integers(-2**31, 2**31, count + 2, dtype=np.int64).astype(np.int32)
+    y = np.full(count + 2, 77, np.int32)
+    d = ctypes.c_void_p()
+    assert lib.ma_buffer_alloc(dev.handle, nbytes + 8, ctypes.byref(d)) == 0
+    try:
+        assert lib.ma_buffer_zero(dev.handle, d, nbytes + 8) == 0
+        assert lib.ma_memcpy_h2d(dev.handle, ctypes.c_void_p(d.value + 4), ctypes.c_void_p(x.ctypes.data + 4), nbytes - 4) == 0
+        assert lib.ma_memcpy_d2h(dev.handle, ctypes.c_void_p(y.ctypes.data), d, nbytes + 4) == 0
+        assert y[0] == 0 and np.array_equal(y[1:count], x[1:count]) and y[count] == 0 and y[count + 1] == 77
+    finally:
+        assert lib.ma_buffer_free(dev.handle, d) == 0
