@@ -3,10 +3,10 @@
 #include <chrono>
 #include <cstring>
 #include <new>
-#include <system_error>
 #include <thread>
 
 #include "bulk_copy.cuh"
+#include "copy_threads.h"
 #include "ma_internal.h"
 
 namespace ma {
@@ -73,22 +73,6 @@ static int copy_threads() {
     return n >= (unsigned)kCopyThreads ? kCopyThreads : 1;
 }
 
-// work(0 .. kCopyThreads-1), one of them on the calling thread; without threads to be had all of them there.
-template <class F>
-static void on_copy_threads(const F& work) {
-    std::thread pool[kCopyThreads];
-    for (int i = 1; i < kCopyThreads; ++i) {
-        try {
-            pool[i] = std::thread(work, i);
-        } catch (const std::system_error&) {
-            work(i);
-        }
-    }
-    work(0);
-    for (int i = 1; i < kCopyThreads; ++i)
-        if (pool[i].joinable()) pool[i].join();
-}
-
 // One filling of the staging buffer, host -> device (to_device) or back, in kCopyPieces pieces.
 static cudaError_t threaded_copy(ma_context* ctx, char* dptr, char* host, size_t bytes, bool to_device) {
     const size_t piece = ((bytes + kCopyPieces - 1) / kCopyPieces + 4095) & ~(size_t)4095;
@@ -105,7 +89,7 @@ static cudaError_t threaded_copy(ma_context* ctx, char* dptr, char* host, size_t
             }
         }
     }
-    on_copy_threads([&](int i) {
+    on_threads<kCopyThreads>([&](int i) {
         cudaError_t e = i == 0 ? cudaSuccess : cudaSetDevice(ctx->device);
         for (int k = i; k < kCopyPieces && size_of(k) > 0 && e == cudaSuccess; k += kCopyThreads) {
             if (to_device) {

@@ -34,3 +34,16 @@ def test_cpp_mirror_host_logic(exe):
 def test_cpp_mirror_on_gpu(exe):
     r = subprocess.run([exe], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0 and "OK" in r.stdout, r.stdout + r.stderr
+
+
+def test_copy_threads_that_cannot_start(tmp_path):
+    """The threads of the large pageable copies: whichever of them cannot be started, and for whatever reason, its
+    part is done once on the calling thread and no exception leaves the C function."""
+    gxx = shutil.which("g++")
+    if gxx is None:
+        pytest.skip("g++ not available")
+    exe = tmp_path / "copy_threads_test"
+    subprocess.run([gxx, "-std=c++17", "-O1", "-pthread", os.path.join(ROOT, "tests", "cpp", "copy_threads_test.cpp"), "-o", str(exe)],
+                   check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
+    assert r.returncode == 0, r.stdout + r.stderr
