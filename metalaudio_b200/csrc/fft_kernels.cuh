@@ -396,7 +396,7 @@ struct C2RParams {
     const float* norm_mid;      // iSTFT: clamped window sums of the interior, indexed by position mod hop
     const float* norm_mid_inv;  // iSTFT: their reciprocals
     const float* norm_edge;     // iSTFT: window sums of the first N positions, then of the last frame's N positions
-                                // (host_tables.h make_edge_tables), or nullptr
+                                // (window_sum_entry), or nullptr
     int32_t* error_flag;        // set to 1 when a bounded wait ran out
     int32_t dependent_launch;   // launched with programmatic stream serialization (see fft_small.cu)
     const float4* window_syn;   // register-ring iSTFT: synthesis window in thread order with 1/N folded in
@@ -770,6 +770,21 @@ MA_HD float window_sum_at(const float* __restrict__ window, int64_t o, int N, in
 // one another those positions see only one end of the signal, and their sums are tabulated: evaluated in
 // place they cost two 64-bit divisions and a chain of loads per sample, which made the CTAs that hold a
 // signal's ends the ones every short batch waited for (8 signals of 332 frames, 4096 points, hop 1024: 69 -> 49 us).
+// The table's entries: [0, N) position o of a signal, which frames 0 .. o/hop cover; [N, 2N) position
+// (frames-1)*hop + u, which only the last frames reach.  Same frame order and floor as window_sum_at.
+MA_HD float window_sum_entry(const float* __restrict__ window, int i, int N, int hop, float floor) {
+    const int u = i < N ? i : i - N;
+    const int top = i < N ? u : u + ((N - 1 - u) / hop) * hop, bottom = i < N ? 0 : u;
+    float acc = 0.f;
+#pragma unroll 8
+    for (int off = top; off >= bottom; off -= hop) {
+        const float w = window ? MA_LDG(window + off) : 1.0f;
+        acc = fmaf(w, w, acc);
+    }
+    if (acc < 1.17549435e-38f) acc = 0.f;
+    return acc > floor ? acc : floor;
+}
+
 MA_HD float window_sum_edge(const C2RParams& p, int64_t o, int N, int hop, int64_t frames) {
     if (p.norm_edge != nullptr && (frames - 1) * hop >= (int64_t)(N - hop))
         return o < (frames - 1) * (int64_t)hop ? MA_LDG(p.norm_edge + o) : MA_LDG(p.norm_edge + N + (o - (frames - 1) * hop));

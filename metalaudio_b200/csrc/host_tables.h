@@ -197,23 +197,4 @@ inline std::vector<float> make_norm_table(const float* window, int n, int hop, f
     return tab;
 }
 
-// Window sums outside the interior, for signals with more frames than overlap one another, in the same order
-// and with the same floor: [0, n) position o of a signal, which frames 0 .. o/hop cover; [n, 2n) position
-// (frames-1)*hop + u, which only the last frames reach.
-inline std::vector<float> make_edge_tables(const float* window, int n, int hop, float floor) {
-    std::vector<float> tab(2 * (size_t)n);
-    for (int i = 0; i < 2 * n; ++i) {
-        const int u = i % n;
-        const int top = i < n ? u : u + ((n - 1 - u) / hop) * hop, bottom = i < n ? 0 : u;
-        float acc = 0.f;
-        for (int off = top; off >= bottom; off -= hop) {
-            const float w = window ? window[off] : 1.0f;
-            acc = std::fma(w, w, acc);
-        }
-        if (acc < 1.17549435e-38f) acc = 0.f;
-        tab[(size_t)i] = acc > floor ? acc : floor;
-    }
-    return tab;
-}
-
 }  // namespace ma

@@ -12,6 +12,13 @@
 
 using namespace ma;
 
+// The table the device fills: window sums of the positions at either end of a signal.
+static std::vector<float> edge_sums(const float* window, int n, int hop, float floor) {
+    std::vector<float> tab(2 * (size_t)n);
+    for (int i = 0; i < 2 * n; ++i) tab[(size_t)i] = window_sum_entry(window, i, n, hop, floor);
+    return tab;
+}
+
 extern "C" {
 
 // Forward R2C of total_frames frames; returns 0 on success, -1 for an unsupported size.
@@ -89,7 +96,7 @@ int emul_istft(int n, int hop, const float* in_a, const float* in_b, long long i
     for (int r = 0; r < hop; ++r) norm[(size_t)(hop + r)] = 1.0f / norm[(size_t)r];
     p.norm_mid = norm.data();
     p.norm_mid_inv = norm.data() + hop;
-    const auto edge = make_edge_tables(window, n, hop, floor);
+    const auto edge = edge_sums(window, n, hop, floor);
     p.norm_edge = edge.data();
     auto syn = make_synthesis_table(window, M);
     p.window_syn = (window != nullptr && !syn.empty()) ? reinterpret_cast<const float4*>(syn.data()) : nullptr;
@@ -173,7 +180,7 @@ int emul_istft_rows(int n, int hop, const float* in_a, const float* in_b, long l
     }
     p.norm_mid = norm.data();
     p.norm_mid_inv = norm.data() + hop;
-    const auto edge = make_edge_tables(window, n, hop, floor);
+    const auto edge = edge_sums(window, n, hop, floor);
     p.norm_edge = edge.data();
     p.twM = twM.data(); p.twN = twN.data();
     int rc = -1;

@@ -121,3 +121,53 @@ def test_large_frames_many_signals_half_layout(device):
     y = fft.istftBatch(spec)
     m = interior(frames, n, hop, w)
     assert o64.rel_rms(y[:, m], x[:, :y.shape[1]][:, m]) <= TOL
+
+
+def _istft_dev(lib, fft, spec, out, floor):
+    import ctypes
+    frames = spec.shape[1]
+    assert lib.ma_istft_dev(fft._h, ctypes.c_void_p(spec.pointer), None, frames, spec.shape[0], ctypes.c_void_p(out.pointer),
+                            out.shape[1], floor, 0) == 0
+
+
+@pytest.mark.parametrize("n,hop,frames", [(4096, 1024, 12), (1024, 16, 200), (512, 160, 30), (4096, 1280, 9), (256, 256, 3)])
+def test_istft_floor_changes_on_one_plan(lib, device, n, hop, frames):
+    """The window sums are tabulated per plan and floor: a plan whose floor changes from call to call gives what the
+    definition gives, at the ends of the signal too (Hann, floor up to 0.1: the outermost samples are divided by it)."""
+    from metalaudio_b200 import FFT, Tensor
+    w = rp.periodic_hann(n)
+    fft = FFT(device, FFT.Config(size=n, hopSize=hop), window=w)
+    rng = np.random.default_rng(n + hop)
+    spec64 = rng.standard_normal((2, frames, n // 2 + 1)) + 1j * rng.standard_normal((2, frames, n // 2 + 1))
+    spec64[..., 0] = spec64[..., 0].real
+    spec64[..., -1] = spec64[..., -1].real
+    half = np.stack([spec64.real, spec64.imag], -1).astype(np.float32)
+    spec, out = Tensor(device, half.shape), Tensor(device, (2, (frames - 1) * hop + n))
+    spec.copy(half)
+    for floor in (0.1, 1e-3, 0.1):
+        _istft_dev(lib, fft, spec, out, floor)
+        device.synchronize()
+        ref = o64.istft(half[..., 0].astype(np.float64) + 1j * half[..., 1], n, hop, w, floor)
+        assert o64.rel_rms(out.toArray(), ref) <= TOL
+    fft.close()
+
+
+def test_first_istft_of_a_plan_with_many_overlaps(lib, device):
+    """A plan's first iSTFT builds the window sums of both ends, 2N positions of up to N/hop frames each.  At 8192
+    points and a hop of 1 that is 6.7e7 terms: 235 ms as a host loop, below a millisecond as a kernel."""
+    import time
+
+    from metalaudio_b200 import FFT, Tensor
+    n, hop, frames = 8192, 1, 8
+    spec, out = Tensor(device, (1, frames, n // 2 + 1, 2)), Tensor(device, (1, (frames - 1) * hop + n))
+    spec.copy(np.zeros(spec.shape, np.float32))
+    took = []
+    for _ in range(3):   # a fresh plan each time; the first one also loads the kernels
+        fft = FFT(device, FFT.Config(size=n, hopSize=hop), window=rp.periodic_hann(n))
+        device.synchronize()
+        t = time.perf_counter()
+        _istft_dev(lib, fft, spec, out, 1e-3)
+        device.synchronize()
+        took.append(time.perf_counter() - t)
+        fft.close()
+    assert min(took[1:]) < 0.06

@@ -31,6 +31,7 @@ def emul():
     deps = [SRC, os.path.join(HERE, "kernel_emulation", "host_cta.h"),
             os.path.join(HERE, "..", "metalaudio_b200", "csrc", "fft_core.cuh"),
             os.path.join(HERE, "..", "metalaudio_b200", "csrc", "fft_kernels.cuh"),
+            os.path.join(HERE, "..", "metalaudio_b200", "csrc", "host_tables.h"),
             os.path.join(HERE, "..", "metalaudio_b200", "csrc", "pconv_tiling.h")]
     if not os.path.exists(OUT) or any(os.path.getmtime(d) > os.path.getmtime(OUT) for d in deps):
         subprocess.run([nvcc, "-std=c++17", "-O1", "-shared", "-Xcompiler", "-fPIC", "-diag-suppress", "20011,20014",
