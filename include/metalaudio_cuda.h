@@ -83,7 +83,14 @@ enum {
 enum { MA_MAG_MAGNITUDE = 0, MA_MAG_POWER = 1, MA_MAG_DB = 2 };
 
 /* Host-side fault injection sites (ma_test_inject_fault). */
-enum { MA_FAULT_ALLOC = 0, MA_FAULT_LAUNCH = 1, MA_FAULT_SYNC = 2, MA_FAULT_DEVICE_LOST = 3 };
+enum {
+    MA_FAULT_ALLOC = 0,
+    MA_FAULT_LAUNCH = 1,
+    MA_FAULT_SYNC = 2,
+    MA_FAULT_DEVICE_LOST = 3,
+    MA_FAULT_RESERVE_SPECTRA = 4, /* ma_pconv_reserve, the coarser partition's spectra */
+    MA_FAULT_RESERVE_BUFFERS = 5  /* ma_pconv_reserve, the buffers for the signals */
+};
 
 typedef struct ma_context ma_context;
 typedef struct ma_fft_plan ma_fft_plan;
@@ -327,8 +334,9 @@ ma_status ma_pconv_step_splits(ma_pconv* pc, int32_t set_to, int32_t* splits);
  * groups' copies in, convolutions and copies out overlap on three streams (see
  * ma_context_reserve_workspace).
  * ma_pconv_reserve also lays the taps out in coarser blocks (up to 4096 samples, at least eight partitions of
- * them) that whole-signal calls on a clear delay line run on: 8 more bytes per tap; without the memory the
- * calls keep block_size.  A non-finite input sample then spoils its whole coarse block besides the reach of the
+ * them) that whole-signal calls on a clear delay line run on: 8 more bytes of device memory per tap, for which
+ * ma_pconv_set_kernels keeps a copy of the taps in host memory until then.  Where the device has no room for
+ * them beside the signals' buffers the calls keep block_size.  A non-finite input sample then spoils its whole coarse block besides the reach of the
  * response, where calls that continue a stream spoil its block of block_size samples. */
 ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len);
 ma_status ma_pconv_process_dev(ma_pconv* pc, const float* in, int64_t len, int64_t in_stride,

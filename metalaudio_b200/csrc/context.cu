@@ -44,6 +44,8 @@ ma_status enter(ma_context* ctx, int site) {
     return MA_OK;
 }
 
+ma_status fault_at(ma_context* ctx, int site) { return ctx->fault_site == site ? injected(ctx) : MA_OK; }
+
 ma_status after_launch(ma_context* ctx) {
     if (ctx != nullptr) ++ctx->launch_seq;
     g_launch_count.fetch_add(1, std::memory_order_relaxed);
@@ -459,7 +461,7 @@ ma_status ma_timing_end(ma_context* ctx, float* milliseconds) {
 }
 
 ma_status ma_test_inject_fault(ma_context* ctx, int32_t site, int32_t cuda_error) {
-    if (ctx == nullptr || site < MA_FAULT_ALLOC || site > MA_FAULT_DEVICE_LOST) return MA_ERR_INVALID_ARGUMENT;
+    if (ctx == nullptr || site < MA_FAULT_ALLOC || site > MA_FAULT_RESERVE_BUFFERS) return MA_ERR_INVALID_ARGUMENT;
     ctx->fault_site = site;
     ctx->fault_error = cuda_error;
     return MA_OK;

@@ -65,6 +65,8 @@ ma_status cuda_fail(cudaError_t e);
 // Returns MA_OK, MA_ERR_DEVICE_LOST, or an injected fault for `site`; makes the
 // context's device current.
 ma_status enter(ma_context* ctx, int site);
+// MA_OK, or the fault injected for `site`.
+ma_status fault_at(ma_context* ctx, int site);
 // Checks the launch error of the kernel just queued and counts it.
 ma_status after_launch(ma_context* ctx);
 

@@ -46,9 +46,8 @@ struct ma_pconv {
     float2* d_y = nullptr;
     // Whole-signal calls that start on a clear delay line need not keep the caller's block size: they run on
     // a coarser partition of the same taps (whole_block), built by ma_pconv_reserve.  Where the caller's own
-    // block is the better one, w_plan and d_hw are plan and d_h.
-    float* d_taps = nullptr;      // [n_irs][taps_stride], kept from set_kernels until the coarse spectra exist
-    int64_t taps_stride = 0;
+    // block is the better one, or the only one there is memory for, w_plan and d_hw are plan and d_h.
+    std::vector<float> h_taps;    // [n_irs][taps], from set_kernels until the coarse spectra and their buffers exist
     int w_block = 0, w_partitions = 0;
     ma_fft_plan* w_plan = nullptr;
     float2* d_hw = nullptr;
@@ -650,12 +649,14 @@ static void free_signal_buffers(ma_pconv* pc) {
     pc->prefix_clear = false;
 }
 
+static int64_t taps_stride(int64_t taps) { return (taps + 3) & ~(int64_t)3; }
+
 // Partition spectra: the taps are the "signals", partitions the "frames" at hop `block`, each
 // frame's samples beyond `block` (and beyond the end of the response) read as zero.
-static ma_status partition_spectra(ma_pconv* pc, ma_fft_plan* plan, int block, int partitions, float2* h) {
+static ma_status partition_spectra(ma_pconv* pc, ma_fft_plan* plan, const float* d_taps, int block, int partitions, float2* h) {
     R2CParams p{};
-    p.in = pc->d_taps;
-    p.signal_stride = pc->taps_stride;
+    p.in = d_taps;
+    p.signal_stride = taps_stride(pc->taps);
     p.frames_per_signal = partitions;
     p.total_frames = (int64_t)partitions * pc->n_irs;
     p.signal_len = pc->taps;
@@ -667,6 +668,13 @@ static ma_status partition_spectra(ma_pconv* pc, ma_fft_plan* plan, int block, i
     p.layout = LAYOUT_HALF_PACKED;
     p.mag_kind = MAG_NONE;
     return launch_r2c_small(plan, p);
+}
+
+// The taps on the device, rows taps_stride apart.
+static ma_status upload_taps(ma_pconv* pc, const float* irs, float* d_taps) {
+    for (int i = 0; i < pc->n_irs; ++i)
+        MA_TRY(copy_h2d(pc->ctx, d_taps + (int64_t)i * taps_stride(pc->taps), irs + (int64_t)i * pc->taps, sizeof(float) * (size_t)pc->taps));
+    return MA_OK;
 }
 
 static void free_coarse(ma_pconv* pc) {
@@ -688,36 +696,63 @@ static int whole_block(int block, int64_t taps) {
     return b;
 }
 
-// Plan and partition spectra of the whole-signal calls.  Without the memory for them the caller's own
-// block size serves those calls too.
-static void build_coarse(ma_pconv* pc) {
+// Without the memory for more the caller's own block size serves the whole-signal calls.
+static void use_own_block(ma_pconv* pc) {
+    free_coarse(pc);
+    pc->w_block = pc->block;
+    pc->w_partitions = pc->partitions;
+    pc->w_plan = pc->plan;
+    pc->d_hw = pc->d_h;
+}
+
+// Plan and partition spectra of the whole-signal calls; MA_ERR_ALLOC without the memory for them.
+static ma_status build_coarse(ma_pconv* pc) {
+    ma_context* ctx = pc->ctx;
     pc->w_block = whole_block(pc->block, pc->taps);
     pc->w_partitions = (int)((pc->taps + pc->w_block - 1) / pc->w_block);
-    if (pc->w_block != pc->block) {
-        ma_context* ctx = pc->ctx;
-        ma_status st = ma_fft_plan_create(ctx, 2 * pc->w_block, nullptr, pc->w_block, &pc->w_plan);
-        if (st == MA_OK) {
-            cudaError_t e = cudaMalloc((void**)&pc->d_hw, sizeof(float2) * (size_t)pc->w_partitions * pc->w_block * (size_t)pc->n_irs);
-            if (e != cudaSuccess) st = cuda_fail(e);
-        }
-        if (st == MA_OK) st = partition_spectra(pc, pc->w_plan, pc->w_block, pc->w_partitions, pc->d_hw);
-        if (st == MA_OK && cudaStreamSynchronize(ctx->stream) != cudaSuccess) st = MA_ERR_CUDA;
-        if (st != MA_OK) free_coarse(pc);
+    if (pc->w_block == pc->block || pc->h_taps.empty()) {
+        use_own_block(pc);
+        return MA_OK;
     }
-    if (pc->w_plan == nullptr) {
-        pc->w_block = pc->block;
-        pc->w_partitions = pc->partitions;
-        pc->w_plan = pc->plan;
-        pc->d_hw = pc->d_h;
+    float* d_taps = nullptr;
+    ma_status st = fault_at(ctx, MA_FAULT_RESERVE_SPECTRA);
+    if (st == MA_OK) st = ma_fft_plan_create(ctx, 2 * pc->w_block, nullptr, pc->w_block, &pc->w_plan);
+    if (st == MA_OK) {
+        cudaError_t e = cudaMalloc((void**)&pc->d_hw, sizeof(float2) * (size_t)pc->w_partitions * pc->w_block * (size_t)pc->n_irs);
+        if (e != cudaSuccess) st = cuda_fail(e);
     }
-    (void)cudaFree(pc->d_taps);
-    pc->d_taps = nullptr;
+    if (st == MA_OK) st = temp_alloc(ctx, sizeof(float) * (size_t)(taps_stride(pc->taps) * pc->n_irs), (void**)&d_taps);
+    if (st == MA_OK) st = upload_taps(pc, pc->h_taps.data(), d_taps);
+    if (st == MA_OK) st = partition_spectra(pc, pc->w_plan, d_taps, pc->w_block, pc->w_partitions, pc->d_hw);
+    temp_free(ctx, d_taps);
+    if (st == MA_OK) {
+        const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+        if (e != cudaSuccess) st = cuda_fail(e);
+    }
+    if (st != MA_OK) free_coarse(pc);
+    return st;
+}
+
+// The timeline and product buffers for outputs of up to `full` samples.  Both partitions share them: the
+// caller's block size serves calls that continue a stream.
+static ma_status alloc_signal_buffers(ma_pconv* pc, int64_t full) {
+    MA_TRY(fault_at(pc->ctx, MA_FAULT_RESERVE_BUFFERS));
+    auto blocks = [&](int b) { return (full + b - 1) / b; };
+    const int64_t own_row = (pc->partitions - 1 + blocks(pc->block)) * pc->block;
+    pc->w_stride = (pc->w_partitions - 1 + blocks(pc->w_block)) * pc->w_block;
+    const int64_t tl_row = own_row > pc->w_stride ? own_row : pc->w_stride;
+    const int64_t own_y = blocks(pc->block) * pc->block, w_y = blocks(pc->w_block) * pc->w_block;
+    cudaError_t e = cudaMalloc((void**)&pc->d_timeline, sizeof(float2) * (size_t)pc->channels * (size_t)tl_row);
+    if (e == cudaSuccess)
+        e = cudaMalloc((void**)&pc->d_y, sizeof(float2) * (size_t)pc->channels * (size_t)(own_y > w_y ? own_y : w_y));
+    if (e == cudaSuccess) return MA_OK;
+    free_signal_buffers(pc);
+    return cuda_fail(e);
 }
 
 static void free_kernel_buffers(ma_pconv* pc) {
     free_coarse(pc);
-    if (pc->d_taps) (void)cudaFree(pc->d_taps);
-    pc->d_taps = nullptr;
+    pc->h_taps = std::vector<float>();
     if (pc->d_h) (void)cudaFree(pc->d_h);
     if (pc->d_ch2ir) (void)cudaFree(pc->d_ch2ir);
     if (pc->d_ring) (void)cudaFree(pc->d_ring);
@@ -838,15 +873,17 @@ ma_status ma_pconv_set_kernels(ma_pconv* pc, const float* irs, int64_t taps, int
         e = cudaMalloc((void**)&pc->d_partial, sizeof(float2) * (size_t)pc->splits * (size_t)C * B);
     if (e != cudaSuccess) st = cuda_fail(e);
     if (st == MA_OK) st = copy_h2d(ctx, pc->d_ch2ir, map.data(), sizeof(int32_t) * (size_t)C);
-    const int64_t tstride = (taps + 3) & ~(int64_t)3;
-    pc->taps_stride = tstride;
-    if (st == MA_OK) {
-        e = cudaMalloc((void**)&pc->d_taps, sizeof(float) * (size_t)(tstride * n_irs));
-        if (e != cudaSuccess) st = cuda_fail(e);
+    float* d_taps = nullptr;
+    if (st == MA_OK) st = temp_alloc(ctx, sizeof(float) * (size_t)(taps_stride(taps) * n_irs), (void**)&d_taps);
+    if (st == MA_OK) st = upload_taps(pc, irs, d_taps);
+    if (st == MA_OK) st = partition_spectra(pc, pc->plan, d_taps, B, P, pc->d_h);
+    temp_free(ctx, d_taps);
+    if (st == MA_OK && whole_block(B, taps) != B) {
+        try {
+            pc->h_taps.assign(irs, irs + taps * n_irs);
+        } catch (const std::bad_alloc&) {  // whole-signal calls keep the caller's block size
+        }
     }
-    for (int i = 0; i < n_irs && st == MA_OK; ++i)
-        st = copy_h2d(ctx, pc->d_taps + (int64_t)i * tstride, irs + (int64_t)i * taps, sizeof(float) * (size_t)taps);
-    if (st == MA_OK) st = partition_spectra(pc, pc->plan, B, P, pc->d_h);
     if (st == MA_OK) st = ma_pconv_reset(pc);
     if (st == MA_OK) {
         cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
@@ -906,21 +943,18 @@ ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len) {
     if (__builtin_add_overflow(max_len, pc->taps - 1, &full)) return MA_ERR_OUTPUT_OVERFLOW;
     MA_CUDA(cudaStreamSynchronize(ctx->stream));
     free_signal_buffers(pc);
-    if (pc->w_plan == nullptr) build_coarse(pc);
-    // both partitions share the buffers: the caller's block size serves calls that continue a stream
-    auto blocks = [&](int b) { return (full + b - 1) / b; };
-    const int64_t own_row = (pc->partitions - 1 + blocks(pc->block)) * pc->block;
-    pc->w_stride = (pc->w_partitions - 1 + blocks(pc->w_block)) * pc->w_block;
-    const int64_t tl_row = own_row > pc->w_stride ? own_row : pc->w_stride;
-    const int64_t own_y = blocks(pc->block) * pc->block, w_y = blocks(pc->w_block) * pc->w_block;
-    cudaError_t e = cudaMalloc((void**)&pc->d_timeline, sizeof(float2) * (size_t)pc->channels * (size_t)tl_row);
-    if (e == cudaSuccess)
-        e = cudaMalloc((void**)&pc->d_y, sizeof(float2) * (size_t)pc->channels * (size_t)(own_y > w_y ? own_y : w_y));
-    if (e != cudaSuccess) {
-        ma_status st = cuda_fail(e);
-        free_signal_buffers(pc);
+    ma_status st = pc->w_plan == nullptr ? build_coarse(pc) : MA_OK;
+    if (st == MA_OK) st = alloc_signal_buffers(pc, full);
+    if (st == MA_ERR_ALLOC && pc->w_plan != pc->plan) {
+        // what the coarse partition takes may be what these buffers lack
+        use_own_block(pc);
+        st = alloc_signal_buffers(pc, full);
+    }
+    if (st != MA_OK) {
+        free_coarse(pc);  // the next call lays the taps out afresh
         return st;
     }
+    pc->h_taps = std::vector<float>();
     pc->reserved_len = max_len;
     return MA_OK;
 }

@@ -366,6 +366,78 @@ def test_step_after_other_library_work_reads_fresh_input(device, lib):
         assert o64.rel_rms(y[i], 0.5 * o64.convolve_full(x[i], h)[:n]) <= TOL
 
 
+def zero_step(lib, device, c, block, channels=1):
+    """One streaming step of silence: the delay line stays zero but no longer counts as clear, so the next
+    whole-signal call runs on the caller's own block size."""
+    from metalaudio_b200 import Tensor
+    t = Tensor(device, (channels, block))
+    t.copy(np.zeros((channels, block), np.float32))
+    assert lib.ma_pconv_step_dev(c._h, ctypes.c_void_p(t.pointer), block, ctypes.c_void_p(t.pointer), block) == 0
+    device.synchronize()
+
+
+@pytest.mark.parametrize("site", ["spectra", "buffers", "both"])
+def test_reserve_without_memory_for_the_coarse_partition(lib, device, site):
+    """ma_pconv_reserve when the coarser partition's spectra, or the signals' buffers beside them, cannot be had:
+    the call succeeds and whole-signal calls run on the caller's block size, with the results of that size.  When the
+    buffers fail on that size too the call reports it, and the next one starts afresh."""
+    from metalaudio_b200 import _lib as L
+    block, taps, length, channels = 64, 3000, 9000, 3
+    rng = np.random.default_rng(31)
+    h = (rng.standard_normal((channels, taps)) * np.exp(-np.arange(taps) / 500.0)).astype(np.float32)
+    x = rng.standard_normal((channels, length)).astype(np.float32)
+
+    def fresh():
+        c = conv(device, block, channels=channels)
+        c.setKernel(h, channelToKernel=list(range(channels)))
+        return c
+    own = fresh()
+    zero_step(lib, device, own, block, channels)
+    ref_own = own.process(x)
+    ref_coarse = fresh().process(x)
+    assert not np.array_equal(ref_own, ref_coarse)
+    c = fresh()
+    assert lib.ma_pconv_reserve(c._h, length) == 0   # a first reservation has the coarse spectra ...
+    if site == "spectra":
+        c = fresh()
+        assert lib.ma_test_inject_fault(device.handle, L.FAULT_RESERVE_SPECTRA, 2) == 0   # cudaErrorMemoryAllocation
+        assert lib.ma_pconv_reserve(c._h, length) == 0
+        assert np.array_equal(c.process(x), ref_own)
+    elif site == "buffers":
+        for c in (c, fresh()):                        # ... and gives them back where a longer one does not fit beside them
+            assert lib.ma_test_inject_fault(device.handle, L.FAULT_RESERVE_BUFFERS, 2) == 0
+            assert lib.ma_pconv_reserve(c._h, 2 * length) == 0
+            assert np.array_equal(c.process(x), ref_own)
+    else:
+        c = fresh()
+        assert lib.ma_test_inject_fault(device.handle, L.FAULT_RESERVE_BUFFERS, 1) == 0   # not a matter of memory
+        assert lib.ma_pconv_reserve(c._h, length) == L.MA_ERR_CUDA
+        assert np.array_equal(c.process(x), ref_coarse)
+    for i in range(channels):
+        assert o64.rel_rms(c.process(x)[i], o64.convolve_full(x[i], h[i])) <= TOL
+    # new taps: the coarse partition again
+    c.setKernel(h, channelToKernel=list(range(channels)))
+    assert np.array_equal(c.process(x), ref_coarse)
+
+
+def test_taps_take_no_device_memory_before_a_reservation(lib, device):
+    """A convolver that only streams holds its spectra, its delay line and nothing else on the device: not the taps,
+    which only ma_pconv_reserve lays out a second time."""
+    import torch
+    block, taps, irs = 64, 65536, 256
+    h = np.random.default_rng(5).standard_normal((irs, taps)).astype(np.float32)
+    c = conv(device, block, channels=irs)
+    c.setKernel(h[:, :64], channelToKernel=list(range(irs)))   # creates the plan and the object
+    free0 = torch.cuda.mem_get_info()[0]
+    c.setKernel(h, channelToKernel=list(range(irs)))           # the temporary copy of the taps joins the pool
+    c.setKernel(h[:, :64], channelToKernel=list(range(irs)))
+    pool = free0 - torch.cuda.mem_get_info()[0]
+    c.setKernel(h, channelToKernel=list(range(irs)))
+    held = free0 - torch.cuda.mem_get_info()[0] - pool
+    need = 2 * 8 * irs * taps                                  # spectra and delay line
+    assert held <= need + (40 << 20)                           # the taps would be 64 MiB more
+
+
 def test_errors(device):
     from metalaudio_b200 import Convolution, ConvolutionError, MetalAudioError
     c = conv(device, 64)
