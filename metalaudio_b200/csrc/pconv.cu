@@ -51,9 +51,11 @@ struct ma_pconv {
     int w_block = 0, w_partitions = 0;
     ma_fft_plan* w_plan = nullptr;
     float2* d_hw = nullptr;
-    int64_t w_stride = 0;         // float2 per channel of the coarse timeline
+    // float2 per channel of the coarse timeline.  The w_partitions - 1 rows in front of each channel's are zero, in stream
+    // order, whenever no call is using the buffer otherwise (clear_prefix).
+    int64_t w_stride = 0;
     bool clear = true;            // every delay-line spectrum a later call can reach, and the tail, are zero
-    bool prefix_clear = false;    // the w_partitions - 1 rows in front of each channel's coarse timeline are zero
+    bool step_captured = false;   // a graph holds steps of this object: its replays fill the delay line unseen
 };
 
 namespace ma {
@@ -646,7 +648,6 @@ static void free_signal_buffers(ma_pconv* pc) {
     pc->d_timeline = nullptr;
     pc->d_y = nullptr;
     pc->reserved_len = 0;
-    pc->prefix_clear = false;
 }
 
 static int64_t taps_stride(int64_t taps) { return (taps + 3) & ~(int64_t)3; }
@@ -733,6 +734,17 @@ static ma_status build_coarse(ma_pconv* pc) {
     return st;
 }
 
+// Zeroes the rows in front of every channel's coarse timeline: after the allocation, and after calls that lay the
+// buffer out by the caller's block size.  Kept as a state of the stream, not of the host, so that recorded calls may
+// be replayed between others.
+static ma_status clear_prefix(ma_pconv* pc) {
+    if (pc->w_partitions == 1) return MA_OK;
+    MA_CUDA(cudaMemset2DAsync(pc->d_timeline, sizeof(float2) * (size_t)pc->w_stride, 0,
+                              sizeof(float2) * (size_t)(pc->w_partitions - 1) * (size_t)pc->w_block, (size_t)pc->channels,
+                              pc->ctx->stream));
+    return MA_OK;
+}
+
 // The timeline and product buffers for outputs of up to `full` samples.  Both partitions share them: the
 // caller's block size serves calls that continue a stream.
 static ma_status alloc_signal_buffers(ma_pconv* pc, int64_t full) {
@@ -745,9 +757,9 @@ static ma_status alloc_signal_buffers(ma_pconv* pc, int64_t full) {
     cudaError_t e = cudaMalloc((void**)&pc->d_timeline, sizeof(float2) * (size_t)pc->channels * (size_t)tl_row);
     if (e == cudaSuccess)
         e = cudaMalloc((void**)&pc->d_y, sizeof(float2) * (size_t)pc->channels * (size_t)(own_y > w_y ? own_y : w_y));
-    if (e == cudaSuccess) return MA_OK;
-    free_signal_buffers(pc);
-    return cuda_fail(e);
+    const ma_status st = e == cudaSuccess ? clear_prefix(pc) : cuda_fail(e);
+    if (st != MA_OK) free_signal_buffers(pc);
+    return st;
 }
 
 static void free_kernel_buffers(ma_pconv* pc) {
@@ -842,6 +854,7 @@ ma_status ma_pconv_set_kernels(ma_pconv* pc, const float* irs, int64_t taps, int
     pc->n_irs = n_irs;
     pc->share = share;
     pc->write_index = 0;
+    pc->step_captured = false;
     // Partition splits of the streaming step: about 5.25 CTAs per SM in all (the multiply-accumulate
     // kernel fits 7 of its 128-thread CTAs on an SM; measured for 512 / 256 / 128 channels of block 256
     // with 512 partitions: 768 CTAs 92 / 53 / 35 us per step, 640 CTAs 99 / 58 / 36 us, 1024 CTAs
@@ -961,31 +974,33 @@ ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len) {
 
 }  // extern "C"
 
-// Once per whole-signal call, before its channel ranges: the rows in front of the coarse timeline.
-static ma_status open_whole(ma_pconv* pc) {
-    if (!pc->clear) pc->prefix_clear = false;  // this call lays the buffer out by the caller's block size
-    if (!pc->clear || pc->prefix_clear || pc->w_partitions == 1) return MA_OK;
-    MA_CUDA(cudaMemset2DAsync(pc->d_timeline, sizeof(float2) * (size_t)pc->w_stride, 0,
-                              sizeof(float2) * (size_t)(pc->w_partitions - 1) * (size_t)pc->w_block, (size_t)pc->channels,
-                              pc->ctx->stream));
-    pc->prefix_clear = true;
-    return MA_OK;
+static bool capturing(const ma_context* ctx) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(ctx->stream, &status) == cudaSuccess && status != cudaStreamCaptureStatusNone;
 }
 
-// ... and after them.  A call pushes ceil((len + taps - 1)/B) >= ceil(len/B) + P - 1 blocks, so the only
-// spectrum of its input that can still be in the delay line is in the slot the next block overwrites.
-static void close_whole(ma_pconv* pc) {
-    pc->write_index = 0;
-    pc->clear = true;
+// Whether a whole-signal call may take the coarse partition, which assumes a delay line of zeros.
+static bool runs_coarse(const ma_pconv* pc) { return pc->clear && !pc->step_captured; }
+
+// Once per whole-signal call, after its channel ranges (`done`: all of them are queued).  A call pushes
+// ceil((len + taps - 1)/B) >= ceil(len/B) + P - 1 blocks, so the only spectrum of its input that can still be in the
+// delay line is in the slot the next block overwrites.  A recorded call has not run yet: it leaves `clear` alone.
+static ma_status close_whole(ma_pconv* pc, bool done) {
+    if (!runs_coarse(pc)) MA_TRY(clear_prefix(pc));
+    if (done) {
+        pc->write_index = 0;
+        if (!capturing(pc->ctx)) pc->clear = true;
+    }
+    return MA_OK;
 }
 
 // Whole-signal convolution of channels [c0, c0 + nc) (nc a multiple of the IR-sharing group): `in`
 // and `out` point at channel c0's rows.  Every buffer of the object is per channel, so a range runs
-// on its own slices between open_whole and close_whole.
+// on its own slices; close_whole follows the last range.
 static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, int64_t len, int64_t in_stride,
                                float* out, int64_t out_stride, int64_t full) {
     ma_context* ctx = pc->ctx;
-    const bool coarse = pc->clear;
+    const bool coarse = runs_coarse(pc);
     ma_fft_plan* plan = coarse ? pc->w_plan : pc->plan;
     const int B = coarse ? pc->w_block : pc->block, P = coarse ? pc->w_partitions : pc->partitions;
     const int64_t T = (full + B - 1) / B;
@@ -995,7 +1010,7 @@ static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, in
     float2* timeline = pc->d_timeline + (int64_t)c0 * tl_stride;
     float2* y = pc->d_y + (int64_t)c0 * T * B;
 
-    // 1. history -> timeline prefix (a clear delay line: zeros since open_whole)
+    // 1. history -> timeline prefix (a clear delay line: zeros, see clear_prefix)
     if (P > 1 && !coarse) {
         const int64_t total = (int64_t)nc * (P - 1) * B;
         int grid = (int)((total + 255) / 256 < (int64_t)ctx->sm_count * 8 ? (total + 255) / 256 : (int64_t)ctx->sm_count * 8);
@@ -1084,10 +1099,9 @@ ma_status ma_pconv_process_dev(ma_pconv* pc, const float* in, int64_t len, int64
     if (__builtin_add_overflow(len, pc->taps - 1, &full)) return MA_ERR_OUTPUT_OVERFLOW;
     if (len > pc->reserved_len) return MA_ERR_INVALID_ARGUMENT;
     if (pc->channels > 1 && (in_stride < len || out_stride < full)) return MA_ERR_INVALID_ARGUMENT;
-    MA_TRY(open_whole(pc));
-    MA_TRY(process_range(pc, 0, pc->channels, in, len, in_stride, out, out_stride, full));
-    close_whole(pc);
-    return MA_OK;
+    const ma_status st = process_range(pc, 0, pc->channels, in, len, in_stride, out, out_stride, full);
+    const ma_status closed = close_whole(pc, st == MA_OK);
+    return st != MA_OK ? st : closed;
 }
 
 // Host form: groups of channels go through the context's three-stage pipeline (copy in, convolve,
@@ -1111,7 +1125,6 @@ ma_status ma_pconv_process_host(ma_pconv* pc, const float* in, int64_t len, int6
     const int group = pc->share;  // channels that must stay together (they share one impulse response)
     const size_t in_row = round256(sizeof(float) * (size_t)len), out_row = round256(sizeof(float) * (size_t)full);
     const bool pinned = is_pinned(in) && is_pinned(out);
-    MA_TRY(open_whole(pc));
     Pipe pp;
     MA_TRY(pipe_open(pp, ctx, pinned, C / group, (in_row + out_row) * (size_t)group, 0));
     const int64_t step = pp.chunk * group;
@@ -1132,8 +1145,8 @@ ma_status ma_pconv_process_host(ma_pconv* pc, const float* in, int64_t len, int6
         pp.after_copy_out(i);
     }
     const ma_status st = pp.finish();
-    if (st == MA_OK) close_whole(pc);
-    return st;
+    const ma_status closed = close_whole(pc, st == MA_OK);
+    return st != MA_OK ? st : closed;
 }
 
 ma_status ma_pconv_step_dev(ma_pconv* pc, const float* in_block, int64_t in_stride, float* out_block,
@@ -1148,6 +1161,7 @@ ma_status ma_pconv_step_dev(ma_pconv* pc, const float* in_block, int64_t in_stri
     if (pc->write_index < 0 || pc->write_index >= P) return MA_ERR_INVALID_PARTITION_STATE;
     const int w = pc->write_index;
     pc->clear = false;
+    if (!pc->step_captured && capturing(ctx)) pc->step_captured = true;
     // The three kernels are chained by programmatic dependent launch: this step's r2c may run
     // beside the previous step's c2r (see fft_small.cu).  That is only sound when the kernel right
     // before this r2c on the stream is that c2r and the two share no data: r2c reads its input

@@ -438,6 +438,109 @@ def test_taps_take_no_device_memory_before_a_reservation(lib, device):
     assert held <= need + (40 << 20)                           # the taps would be 64 MiB more
 
 
+class Recorded:
+    """Calls on the library's stream recorded into a CUDA graph."""
+
+    def __init__(self, lib, device, calls):
+        import torch
+        self.stream = torch.cuda.ExternalStream(lib.ma_context_stream(device.handle))
+        self.graph = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(self.stream):
+            self.graph.capture_begin(capture_error_mode="relaxed")
+            try:
+                calls()
+            finally:
+                self.graph.capture_end()
+
+    def replay(self):
+        import torch
+        with torch.cuda.stream(self.stream):
+            self.graph.replay()
+
+
+def test_recorded_whole_signal_calls_and_streaming_between_them(lib, device):
+    """Whole-signal calls recorded into a graph, on a clear delay line: neither the recording (nothing runs then) nor
+    calls that continue a stream, before or between replays, leave rows behind that the next call takes for the zeros
+    in front of the signal."""
+    from metalaudio_b200 import Tensor
+    block, taps, length, channels = 64, 3000, 9000, 2
+    full = length + taps - 1
+    rng = np.random.default_rng(51)
+    h = (rng.standard_normal(taps) * np.exp(-np.arange(taps) / 500.0)).astype(np.float32)
+    x = rng.standard_normal((channels, length)).astype(np.float32)
+    ref = np.stack([o64.convolve_full(x[i], h) for i in range(channels)])
+    c = conv(device, block, channels=channels)
+    c.setKernel(h)
+    tin, out, blk = Tensor(device, x.shape), Tensor(device, (channels, full)), Tensor(device, (channels, block))
+    tin.copy(x)
+    blk.copy(np.full((channels, block), 50.0, np.float32))
+    assert lib.ma_pconv_reserve(c._h, length) == 0
+
+    def whole():
+        assert lib.ma_pconv_process_dev(c._h, ctypes.c_void_p(tin.pointer), length, length, ctypes.c_void_p(out.pointer), full) == 0
+
+    def stream():   # fills the delay line, and the buffer by the caller's block size; clear afterwards
+        for _ in range(3):
+            assert lib.ma_pconv_step_dev(c._h, ctypes.c_void_p(blk.pointer), block, ctypes.c_void_p(out.pointer), full) == 0
+        whole()
+
+    def check(call):
+        out.zero()
+        call()
+        device.synchronize()
+        y = out.toArray()
+        assert all(o64.rel_rms(y[i], ref[i]) <= TOL for i in range(channels))
+    check(whole)
+    stream()
+    g = Recorded(lib, device, whole)
+    check(whole)
+    check(g.replay)
+    stream()
+    check(g.replay)
+    check(whole)
+    check(g.replay)
+
+
+def test_recorded_steps_fill_the_delay_line(lib, device):
+    """A graph of one turn of the delay line (as many steps as partitions): after its replay a whole-signal call
+    continues that stream, as after the same steps called directly, also when the object was reset in between."""
+    from metalaudio_b200 import Tensor
+    block, taps, length = 64, 1500, 4000
+    parts, full = -(-taps // block), length + taps - 1
+    rng = np.random.default_rng(52)
+    h = (rng.standard_normal(taps) * np.exp(-np.arange(taps) / 300.0)).astype(np.float32)
+    past = rng.standard_normal((1, parts * block)).astype(np.float32)
+    x = rng.standard_normal((1, length)).astype(np.float32)
+    tin, tpast, out, blk = Tensor(device, x.shape), Tensor(device, past.shape), Tensor(device, (1, full)), Tensor(device, past.shape)
+    tin.copy(x)
+    tpast.copy(past)
+    results = []
+    for recorded in (False, True):
+        c = conv(device, block)
+        c.setKernel(h)
+        assert lib.ma_pconv_reserve(c._h, length) == 0
+
+        def steps():
+            for b in range(parts):
+                assert lib.ma_pconv_step_dev(c._h, ctypes.c_void_p(tpast.pointer + 4 * b * block), past.shape[1],
+                                             ctypes.c_void_p(blk.pointer + 4 * b * block), past.shape[1]) == 0
+        steps()
+        assert lib.ma_pconv_reset(c._h) == 0
+        if recorded:
+            g = Recorded(lib, device, steps)
+            assert lib.ma_pconv_reset(c._h) == 0
+            g.replay()
+        else:
+            steps()
+        assert lib.ma_pconv_process_dev(c._h, ctypes.c_void_p(tin.pointer), length, length, ctypes.c_void_p(out.pointer), full) == 0
+        device.synchronize()
+        results.append((blk.toArray(), out.toArray()))
+    assert np.array_equal(results[0][0], results[1][0])
+    assert np.array_equal(results[0][1], results[1][1])
+    alone = o64.convolve_full(x[0], h)
+    assert o64.rel_rms(results[0][1][0], alone) > 0.05   # the stream before it is heard
+
+
 def test_errors(device):
     from metalaudio_b200 import Convolution, ConvolutionError, MetalAudioError
     c = conv(device, 64)
