@@ -89,7 +89,9 @@ enum {
     MA_FAULT_SYNC = 2,
     MA_FAULT_DEVICE_LOST = 3,
     MA_FAULT_RESERVE_SPECTRA = 4, /* ma_pconv_reserve, the coarser partition's spectra */
-    MA_FAULT_RESERVE_BUFFERS = 5  /* ma_pconv_reserve, the buffers for the signals */
+    MA_FAULT_RESERVE_BUFFERS = 5, /* ma_pconv_reserve, the buffers for the signals */
+    MA_FAULT_BIQUAD_LADDER = 6,   /* ma_biquad_set_coefficients, the tables of the time splits */
+    MA_FAULT_BIQUAD_MAP = 7       /* ma_biquad_set_coefficients, the channel map */
 };
 
 typedef struct ma_context ma_context;

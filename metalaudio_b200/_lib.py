@@ -98,7 +98,8 @@ MA_OK = 0
  MA_ERR_INPUT_SIZE_MISMATCH) = range(1, 19)
 LAYOUT_HALF_INTERLEAVED, LAYOUT_FULL_SPLIT, LAYOUT_HALF_PACKED, LAYOUT_HALF_POLAR = 0, 1, 2, 3
 MAG_MAGNITUDE, MAG_POWER, MAG_DB = 0, 1, 2
-FAULT_ALLOC, FAULT_LAUNCH, FAULT_SYNC, FAULT_DEVICE_LOST, FAULT_RESERVE_SPECTRA, FAULT_RESERVE_BUFFERS = range(6)
+(FAULT_ALLOC, FAULT_LAUNCH, FAULT_SYNC, FAULT_DEVICE_LOST, FAULT_RESERVE_SPECTRA, FAULT_RESERVE_BUFFERS,
+ FAULT_BIQUAD_LADDER, FAULT_BIQUAD_MAP) = range(8)
 
 _lib = None
 

@@ -26,6 +26,7 @@
 #include <cmath>
 #include <new>
 #include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "ma_internal.h"
@@ -557,8 +558,11 @@ ma_status ma_biquad_create(ma_context* ctx, int32_t n_channels, int32_t n_sectio
     bq->per = n_sections >= kBqLongFrom ? kBqPerLong : kBqPerShort;
     cudaError_t e = cudaMalloc((void**)&bq->d_state, sizeof(float2) * (size_t)n_channels * n_sections);
     if (e == cudaSuccess) e = cudaMemsetAsync(bq->d_state, 0, sizeof(float2) * (size_t)n_channels * n_sections, ctx->stream);  // ordered before the first kernel of the context
-    if (e == cudaSuccess && split_max_chunks(bq) >= kBqSplitFrom)
-        e = cudaMalloc((void**)&bq->d_ends, sizeof(double2) * (size_t)(2 * ctx->sm_count) * n_sections);
+    if (e == cudaSuccess && split_max_chunks(bq) >= kBqSplitFrom &&
+        cudaMalloc((void**)&bq->d_ends, sizeof(double2) * (size_t)(2 * ctx->sm_count) * n_sections) != cudaSuccess) {
+        (void)cudaGetLastError();  // without it the cascade is not split over time
+        bq->d_ends = nullptr;
+    }
     if (e != cudaSuccess) {
         ma_biquad_destroy(bq);
         return cuda_fail(e);
@@ -591,7 +595,7 @@ ma_status ma_biquad_set_coefficients(ma_biquad* bq, const float* coeffs, int32_t
     std::vector<double> tables((size_t)n_sets * bq->sections * kBqTable);
     for (int64_t i = 0; i < (int64_t)n_sets * bq->sections; ++i) build_table(coeffs + 5 * i, tables.data() + kBqTable * i, bq->per);
     std::vector<double> ladder;
-    if (split_max_chunks(bq) >= kBqSplitFrom) {
+    if (bq->d_ends != nullptr) {
         const size_t per_set = (size_t)kBqLadder * 4 * bq->sections * bq->sections;
         ladder.resize(per_set * n_sets);
         bool ok = true;
@@ -600,23 +604,33 @@ ma_status ma_biquad_set_coefficients(ma_biquad* bq, const float* coeffs, int32_t
         if (!ok) ladder.clear();
     }
     MA_TRY(ma_context_sync(ctx, 30.0));  // nothing in flight may still read the old tables
-    if (bq->d_tables) (void)cudaFree(bq->d_tables);
-    if (bq->d_map) (void)cudaFree(bq->d_map);
-    if (bq->d_ladder) (void)cudaFree(bq->d_ladder);
-    bq->d_tables = nullptr;
-    bq->d_map = nullptr;
-    bq->d_ladder = nullptr;
-    MA_CUDA(cudaMalloc((void**)&bq->d_tables, tables.size() * sizeof(double)));
-    MA_TRY(copy_h2d(ctx, bq->d_tables, tables.data(), tables.size() * sizeof(double)));
-    if (!ladder.empty()) {
-        MA_CUDA(cudaMalloc((void**)&bq->d_ladder, ladder.size() * sizeof(double)));
-        MA_TRY(copy_h2d(ctx, bq->d_ladder, ladder.data(), ladder.size() * sizeof(double)));
+    // The new arrays replace the old ones when all of them are there: a call that fails leaves the coefficients as they were.
+    double *d_tables = nullptr, *d_ladder = nullptr;
+    int32_t* d_map = nullptr;
+    auto upload = [&](const void* host, size_t bytes, auto** dptr) {
+        MA_CUDA(cudaMalloc((void**)dptr, bytes));
+        return copy_h2d(ctx, *dptr, host, bytes);
+    };
+    ma_status st = upload(tables.data(), tables.size() * sizeof(double), &d_tables);
+    if (st == MA_OK && !ladder.empty()) {
+        st = fault_at(ctx, MA_FAULT_BIQUAD_LADDER);
+        if (st == MA_OK) st = upload(ladder.data(), ladder.size() * sizeof(double), &d_ladder);
+        if (st == MA_ERR_ALLOC && d_ladder == nullptr) st = MA_OK;  // without the ladder the cascade is not split over time
     }
-    if (channel_to_set != nullptr) {
-        MA_CUDA(cudaMalloc((void**)&bq->d_map, sizeof(int32_t) * (size_t)bq->channels));
-        MA_TRY(copy_h2d(ctx, bq->d_map, channel_to_set, sizeof(int32_t) * (size_t)bq->channels));
+    if (st == MA_OK && channel_to_set != nullptr) {
+        st = fault_at(ctx, MA_FAULT_BIQUAD_MAP);
+        if (st == MA_OK) st = upload(channel_to_set, sizeof(int32_t) * (size_t)bq->channels, &d_map);
     }
-    bq->sets = n_sets;
+    if (st == MA_OK) {
+        std::swap(bq->d_tables, d_tables);
+        std::swap(bq->d_ladder, d_ladder);
+        std::swap(bq->d_map, d_map);
+        bq->sets = n_sets;
+    }
+    if (d_tables) (void)cudaFree(d_tables);
+    if (d_ladder) (void)cudaFree(d_ladder);
+    if (d_map) (void)cudaFree(d_map);
+    MA_TRY(st);
     return ma_context_sync(ctx, 30.0);
 }
 

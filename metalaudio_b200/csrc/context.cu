@@ -461,7 +461,7 @@ ma_status ma_timing_end(ma_context* ctx, float* milliseconds) {
 }
 
 ma_status ma_test_inject_fault(ma_context* ctx, int32_t site, int32_t cuda_error) {
-    if (ctx == nullptr || site < MA_FAULT_ALLOC || site > MA_FAULT_RESERVE_BUFFERS) return MA_ERR_INVALID_ARGUMENT;
+    if (ctx == nullptr || site < MA_FAULT_ALLOC || site > MA_FAULT_BIQUAD_MAP) return MA_ERR_INVALID_ARGUMENT;
     ctx->fault_site = site;
     ctx->fault_error = cuda_error;
     return MA_OK;

@@ -224,3 +224,45 @@ def test_time_splits_match_float64(device, lib, channels, sections, tiles, extra
             assert np.max(np.abs(z - zref)) <= 1e-4 * max(1.0, float(np.max(np.abs(zref))))
     finally:
         lib.ma_biquad_destroy(h)
+
+
+def test_coefficients_that_cannot_be_stored(device, lib):
+    """ma_biquad_set_coefficients without the memory for one of its arrays: a channel map that cannot be had leaves the
+    old coefficients of every channel in force; the tables of the time splits are only for speed, without them the call
+    succeeds and the cascade runs unsplit."""
+    from metalaudio_b200 import Tensor
+    from metalaudio_b200 import _lib as L
+    channels, length = 3, 70 * 8192
+    x = np.random.default_rng(9).standard_normal((channels, length)).astype(np.float32)
+    designs = [rp.biquad_coefficients("peaking", f, 48000.0, 1.0, 6.0) for f in (100.0, 1000.0, 5000.0, 9000.0)]
+    old = np.array(designs[:2], np.float32)[:, None, :]
+    new = np.array(designs[2:], np.float32)[:, None, :]
+    old_map, new_map = np.array([0, 1, 0], np.int32), np.array([1, 0, 1], np.int32)
+    vp = lambda a: a.ctypes.data_as(ctypes.c_void_p)
+    h = ctypes.c_void_p()
+    assert lib.ma_biquad_create(device.handle, channels, 1, ctypes.byref(h)) == 0
+    tin, tout = Tensor(device, x.shape), Tensor(device, x.shape)
+    tin.copy(x)
+
+    def run(coefs, of_channel):
+        before = lib.ma_kernel_launch_count()
+        assert lib.ma_biquad_reset(h) == 0
+        assert lib.ma_biquad_process_dev(h, ctypes.c_void_p(tin.pointer), length, ctypes.c_void_p(tout.pointer), length, length) == 0
+        device.synchronize()
+        for c in range(channels):
+            ref, _ = rp.biquad_process(x[c].astype(np.float64), coefs[of_channel[c], 0], dtype=np.float64)
+            assert o64.rel_rms(tout.toArray()[c], ref) <= TOL
+        return lib.ma_kernel_launch_count() - before
+    try:
+        assert lib.ma_biquad_set_coefficients(h, vp(old), 2, vp(old_map)) == 0
+        assert run(old, old_map) == 2      # split: end states, then chunks
+        assert lib.ma_test_inject_fault(device.handle, L.FAULT_BIQUAD_MAP, 2) == 0   # cudaErrorMemoryAllocation
+        assert lib.ma_biquad_set_coefficients(h, vp(new), 2, vp(new_map)) == L.MA_ERR_ALLOC
+        assert run(old, old_map) == 2
+        assert lib.ma_test_inject_fault(device.handle, L.FAULT_BIQUAD_LADDER, 2) == 0
+        assert lib.ma_biquad_set_coefficients(h, vp(new), 2, vp(new_map)) == 0
+        assert run(new, new_map) == 1
+        assert lib.ma_biquad_set_coefficients(h, vp(new), 2, vp(new_map)) == 0
+        assert run(new, new_map) == 2
+    finally:
+        lib.ma_biquad_destroy(h)
