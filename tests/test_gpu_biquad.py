@@ -266,3 +266,29 @@ def test_coefficients_that_cannot_be_stored(device, lib):
         assert run(new, new_map) == 2
     finally:
         lib.ma_biquad_destroy(h)
+
+
+def test_time_splits_of_very_long_channels(device, lib):
+    """74 channels, the most that are split, so long that a chunk holds more than 511 tiles: still split, and the last
+    chunk's samples are the filter's."""
+    import torch
+    channels, sections, length = 74, 3, 4 * 513 * 4096 - 77
+    coef = np.stack([rp.biquad_coefficients("lowpass", 200.0, 48000.0, 4.0, 0.0), rp.biquad_coefficients("peaking", 40.0, 48000.0, 8.0, 9.0),
+                     rp.biquad_coefficients("highpass", 30.0, 48000.0, 0.7, 0.0)]).astype(np.float32)
+    x = torch.rand((channels, length), device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)) * 2.0 - 1.0
+    picked = {c: x[c].cpu().numpy().astype(np.float64) for c in (0, 73)}
+    torch.cuda.synchronize()
+    h = ctypes.c_void_p()
+    assert lib.ma_biquad_create(device.handle, channels, sections, ctypes.byref(h)) == 0
+    try:
+        assert lib.ma_biquad_set_coefficients(h, coef.ctypes.data_as(ctypes.c_void_p), 1, None) == 0
+        before = lib.ma_kernel_launch_count()
+        assert lib.ma_biquad_process_dev(h, ctypes.c_void_p(x.data_ptr()), length, ctypes.c_void_p(x.data_ptr()), length, length) == 0
+        assert lib.ma_kernel_launch_count() - before == 2   # end states, then chunks
+        device.synchronize(30)
+        for c, y in picked.items():
+            for s in range(sections):
+                y, _ = rp.biquad_process(y, coef[s], dtype=np.float64)
+            assert o64.rel_rms(x[c].cpu().numpy(), y) <= TOL
+    finally:
+        lib.ma_biquad_destroy(h)
