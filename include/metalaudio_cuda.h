@@ -336,12 +336,13 @@ ma_status ma_pconv_step_splits(ma_pconv* pc, int32_t set_to, int32_t* splits);
  * groups' copies in, convolutions and copies out overlap on three streams (see
  * ma_context_reserve_workspace).
  * ma_pconv_reserve also lays the taps out in coarser blocks (up to 4096 samples, at least eight partitions of
- * them) that whole-signal calls on a clear delay line run on: 8 more bytes of device memory per tap, for which
+ * them) that whole-signal calls on a clear delay line run on: 12 more bytes of device memory per tap, for which
  * ma_pconv_set_kernels keeps a copy of the taps in host memory until then.  Where the device has no room for
- * them beside the signals' buffers the calls keep block_size.  Calls recorded by a stream capture: a whole-signal call
- * is recorded for the delay line as it is then, clear or not, and is to be replayed on such a one; once steps have
- * been recorded every whole-signal call keeps block_size, since replays fill the delay line unseen.  A non-finite input sample then spoils its whole coarse block besides the reach of the
- * response, where calls that continue a stream spoil its block of block_size samples. */
+ * them beside the signals' buffers the calls keep block_size.  A non-finite input sample spoils the outputs that its
+ * block of block_size samples reaches, on either route.
+ * Calls recorded by a stream capture: a whole-signal call is recorded for the delay line as it is then, clear or
+ * not, and is to be replayed on such a one; once steps have been recorded every whole-signal call keeps block_size,
+ * since replays fill the delay line unseen. */
 ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len);
 ma_status ma_pconv_process_dev(ma_pconv* pc, const float* in, int64_t len, int64_t in_stride,
                                float* out, int64_t out_stride);

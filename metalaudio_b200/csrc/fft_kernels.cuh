@@ -34,6 +34,8 @@ struct R2CParams {
     const float2* twM;          // stage twiddle tables of FftPlan<M> (fft_core.cuh layout)
     int32_t bulk_ok;            // frame starts and length are 16-byte multiples: bulk async staging allowed
     int32_t* error_flag;        // set to 1 when a bounded wait ran out
+    int32_t* marks;             // the convolution's blocks: marks[signal] = mark where a sample is not finite; nullptr: no look
+    int32_t mark;
     int32_t dependent_launch;   // launched with programmatic stream serialization (see fft_small.cu)
     const float2* twN;          // Hermitian-step twiddles exp(-2 pi i k / N): [k], k <= M/2, or for
                                 // plan_pairable<M>() the table [k][j] = W_N^(j + k*NL), j <= NL/2
@@ -303,6 +305,14 @@ MA_HD void r2c_body(const R2CParams& p, Cta& cta, float2* smem) {
                 if (i0 + 1 < valid) x1 = MA_LDG(src + i0 + 1);
                 const float2 w = p.window != nullptr ? MA_LDG(window2 + (t + q * T)) : make_float2(1.f, 1.f);
                 v[q] = make_float2(x0 * w.x, x1 * w.y);
+            }
+        }
+        if constexpr (HALF || LAYOUT < 0) {  // the kernels the convolution's blocks take
+            if (p.marks != nullptr) {
+                float2 z = make_float2(0.f, 0.f);  // stays zero as long as every sample is finite
+#pragma unroll
+                for (int q = 0; q < (HALF ? R / 2 : R); ++q) z = pfma(v[q], make_float2(0.f, 0.f), z);
+                if (active && !(z.x + z.y == 0.f)) p.marks[s] = p.mark;
             }
         }
 

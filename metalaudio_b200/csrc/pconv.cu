@@ -48,6 +48,9 @@ struct ma_pconv {
     // a coarser partition of the same taps (whole_block), built by ma_pconv_reserve.  Where the caller's own
     // block is the better one, or the only one there is memory for, w_plan and d_hw are plan and d_h.
     std::vector<float> h_taps;    // [n_irs][taps], from set_kernels until the coarse spectra and their buffers exist
+    float* d_taps = nullptr;      // [n_irs][taps_stride], beside the coarse spectra (pconv_rescue_kernel)
+    int32_t* d_marks = nullptr;   // [channels]: the call that last met a non-finite sample in the channel
+    int32_t mark = 0;             // number of the latest coarse call
     int w_block = 0, w_partitions = 0;
     ma_fft_plan* w_plan = nullptr;
     float2* d_hw = nullptr;
@@ -681,8 +684,12 @@ static ma_status upload_taps(ma_pconv* pc, const float* irs, float* d_taps) {
 static void free_coarse(ma_pconv* pc) {
     if (pc->w_plan && pc->w_plan != pc->plan) (void)ma_fft_plan_destroy(pc->w_plan);
     if (pc->d_hw && pc->d_hw != pc->d_h) (void)cudaFree(pc->d_hw);
+    if (pc->d_taps) (void)cudaFree(pc->d_taps);
+    if (pc->d_marks) (void)cudaFree(pc->d_marks);
     pc->w_plan = nullptr;
     pc->d_hw = nullptr;
+    pc->d_taps = nullptr;
+    pc->d_marks = nullptr;
 }
 
 // Block size of whole-signal calls.  The multiply-accumulate costs one complex product per output bin and
@@ -695,6 +702,131 @@ static int whole_block(int block, int64_t taps) {
     int b = block;
     while (b < kWholeBlock && 2 * (int64_t)b * kWholePartitions <= taps) b *= 2;
     return b;
+}
+
+// ---- non-finite samples in a coarse whole-signal call
+//
+// A transform turns one non-finite sample into a non-finite block, so on the coarse partition (blocks of W, PW of them)
+// output block j is lost when input blocks j - PW .. j hold one, on the caller's own (B, P) when blocks j - P .. j do.
+// Outputs that only the coarse blocks lose are computed here from the samples themselves, so that such a sample spoils
+// what it always did.  The forward transforms mark the channels they met one in; without a mark the kernel returns after
+// a look at the marks.  It costs such a call 1.5 us, launched early behind the inverse transform (4 us plainly).  A
+// marked channel costs a scan of its samples and `taps` multiply-adds for each of at most 3 W outputs per non-finite
+// sample: 512 channels x 2^20 samples, 131072 taps 7.3 ms clean, 9.3 ms with one such sample, 131 ms with one in every
+// channel (the caller's own block of 256 takes 64 ms in every case).
+struct RescueParams {
+    const float* in;
+    int64_t len, in_stride;
+    const float* taps;           // [n_irs][taps_stride]
+    int64_t n_taps, taps_stride;
+    const int32_t* ch2ir;
+    float* out;
+    int64_t out_stride, full;
+    const int32_t* marks;        // [channels]: `mark` where this call met a non-finite sample
+    int32_t mark;
+    int channels;
+    int block, coarse;           // B, W (both powers of two, B <= W)
+    int64_t reach, coarse_reach; // P * B, PW * W
+};
+constexpr int kRescueThreads = 256, kRescueOutputs = 4 * kRescueThreads, kRescueTaps = 256;
+constexpr int kRescueWords = (kRescueOutputs + kWholeBlock) / 32;
+
+__device__ __forceinline__ bool not_finite(float x) { return !(fabsf(x) <= 3.402823466e38f); }
+
+__global__ void __launch_bounds__(kRescueThreads) pconv_rescue_kernel(const RescueParams p) {
+    __shared__ uint32_t bad[kRescueWords];   // samples from the chunk's first output position on
+    __shared__ int64_t before;               // the last non-finite sample in front of it, or -1
+    __shared__ __align__(16) float xs[kRescueOutputs + kRescueTaps];
+    __shared__ __align__(16) float hs[kRescueTaps];
+    const int tid = threadIdx.x;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // launched behind the inverse transform (programmatic)
+    bool mine = false;
+    for (int c = tid; c < p.channels; c += kRescueThreads) mine |= p.marks[c] == p.mark;
+    if (!__syncthreads_or(mine)) return;
+    const int64_t chunks = (p.full + kRescueOutputs - 1) / kRescueOutputs;
+    for (int c = 0; c < p.channels; ++c) {
+        if (p.marks[c] != p.mark) continue;
+        const float* x = p.in + c * p.in_stride;
+        const float* h = p.taps + (int64_t)p.ch2ir[c] * p.taps_stride;
+        // channels that lose the same positions, as when all stop at once, still meet different CTAs
+        for (int64_t chunk = (blockIdx.x + 61u * (unsigned)c) % gridDim.x; chunk < chunks; chunk += gridDim.x) {
+            const int64_t o0 = chunk * kRescueOutputs;
+            const int64_t last_o = (o0 + kRescueOutputs < p.full ? o0 + kRescueOutputs : p.full) - 1;
+            // samples that the chunk's coarse blocks depend on: [lo, o0) and [o0, hi)
+            const int64_t lo = (o0 & -(int64_t)p.coarse) - p.coarse_reach;
+            const int64_t hi = (last_o & -(int64_t)p.coarse) + p.coarse;
+            __syncthreads();  // the previous chunk's readers are done
+            if (tid == 0) before = -1;
+            for (int w = tid; w < kRescueWords; w += kRescueThreads) bad[w] = 0;
+            __syncthreads();
+            int64_t last = -1;
+            for (int64_t s = (lo > 0 ? lo : 0) + tid; s < hi && s < p.len; s += kRescueThreads) {
+                if (!not_finite(x[s])) continue;
+                if (s < o0) last = s;
+                else atomicOr(&bad[(s - o0) >> 5], 1u << ((s - o0) & 31));
+            }
+            if (last >= 0) atomicMax((long long*)&before, (long long)last);
+            __syncthreads();
+            // the last non-finite sample in front of `end`, which lies in (o0, hi]
+            auto last_before = [&](int64_t end) {
+                int bits = (int)(end - o0);
+                int w = (bits - 1) >> 5;
+                uint32_t word = bad[w] & (0xffffffffu >> (31 - ((bits - 1) & 31)));
+                while (word == 0 && w > 0) word = bad[--w];
+                return word != 0 ? o0 + 32 * w + 31 - __clz(word) : before;
+            };
+            bool need[4], any = false;
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int64_t o = o0 + 4 * tid + r;
+                need[r] = false;
+                if (o < p.full) {
+                    const int64_t j = o & -(int64_t)p.coarse, i = o & -(int64_t)p.block;
+                    const int64_t lost = last_before(j + p.coarse), lost_anyway = last_before(i + p.block);
+                    need[r] = lost >= 0 && lost >= j - p.coarse_reach && !(lost_anyway >= 0 && lost_anyway >= i - p.reach);
+                }
+                any |= need[r];
+            }
+            if (!__syncthreads_or(any)) continue;
+            double sum[4] = {0.0, 0.0, 0.0, 0.0};
+            for (int64_t n0 = 0; n0 < p.n_taps && n0 <= last_o; n0 += kRescueTaps) {
+                const int count = p.n_taps - n0 < kRescueTaps ? (int)(p.n_taps - n0) : kRescueTaps;
+                __syncthreads();
+                if (tid < count) hs[tid] = h[n0 + tid];
+                const int64_t first = o0 - n0 - kRescueTaps;  // sample of xs[0]
+                for (int k = tid; k < kRescueOutputs + kRescueTaps; k += kRescueThreads) {
+                    const int64_t s = first + k;
+                    xs[k] = s >= 0 && s < p.len ? x[s] : 0.f;
+                }
+                __syncthreads();
+                float part[4] = {0.f, 0.f, 0.f, 0.f};
+                const float* const xo = xs + kRescueTaps + 4 * tid;  // output 4*tid at tap 0
+                float4 hi4 = *reinterpret_cast<const float4*>(xo);
+                int n = 0;
+                for (; n + 4 <= count; n += 4) {  // a window of eight samples: four outputs, four taps
+                    const float4 lo4 = *reinterpret_cast<const float4*>(xo - n - 4), h4 = *reinterpret_cast<const float4*>(hs + n);
+                    const float win[8] = {lo4.x, lo4.y, lo4.z, lo4.w, hi4.x, hi4.y, hi4.z, hi4.w};
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        part[r] = fmaf(h4.x, win[4 + r], part[r]);
+                        part[r] = fmaf(h4.y, win[3 + r], part[r]);
+                        part[r] = fmaf(h4.z, win[2 + r], part[r]);
+                        part[r] = fmaf(h4.w, win[1 + r], part[r]);
+                    }
+                    hi4 = lo4;
+                }
+                for (; n < count; ++n) {
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) part[r] = fmaf(hs[n], xo[r - n], part[r]);
+                }
+#pragma unroll
+                for (int r = 0; r < 4; ++r) sum[r] += (double)part[r];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+                if (need[r]) p.out[c * p.out_stride + o0 + 4 * tid + r] = (float)sum[r];
+        }
+    }
 }
 
 // Without the memory for more the caller's own block size serves the whole-signal calls.
@@ -715,17 +847,17 @@ static ma_status build_coarse(ma_pconv* pc) {
         use_own_block(pc);
         return MA_OK;
     }
-    float* d_taps = nullptr;
     ma_status st = fault_at(ctx, MA_FAULT_RESERVE_SPECTRA);
     if (st == MA_OK) st = ma_fft_plan_create(ctx, 2 * pc->w_block, nullptr, pc->w_block, &pc->w_plan);
     if (st == MA_OK) {
         cudaError_t e = cudaMalloc((void**)&pc->d_hw, sizeof(float2) * (size_t)pc->w_partitions * pc->w_block * (size_t)pc->n_irs);
+        if (e == cudaSuccess) e = cudaMalloc((void**)&pc->d_taps, sizeof(float) * (size_t)(taps_stride(pc->taps) * pc->n_irs));
+        if (e == cudaSuccess) e = cudaMalloc((void**)&pc->d_marks, sizeof(int32_t) * (size_t)pc->channels);
+        if (e == cudaSuccess) e = cudaMemsetAsync(pc->d_marks, 0, sizeof(int32_t) * (size_t)pc->channels, ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(e);
     }
-    if (st == MA_OK) st = temp_alloc(ctx, sizeof(float) * (size_t)(taps_stride(pc->taps) * pc->n_irs), (void**)&d_taps);
-    if (st == MA_OK) st = upload_taps(pc, pc->h_taps.data(), d_taps);
-    if (st == MA_OK) st = partition_spectra(pc, pc->w_plan, d_taps, pc->w_block, pc->w_partitions, pc->d_hw);
-    temp_free(ctx, d_taps);
+    if (st == MA_OK) st = upload_taps(pc, pc->h_taps.data(), pc->d_taps);
+    if (st == MA_OK) st = partition_spectra(pc, pc->w_plan, pc->d_taps, pc->w_block, pc->w_partitions, pc->d_hw);
     if (st == MA_OK) {
         const cudaError_t e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(e);
@@ -982,6 +1114,11 @@ static bool capturing(const ma_context* ctx) {
 // Whether a whole-signal call may take the coarse partition, which assumes a delay line of zeros.
 static bool runs_coarse(const ma_pconv* pc) { return pc->clear && !pc->step_captured; }
 
+// Once per whole-signal call, before its channel ranges.
+static void open_whole(ma_pconv* pc) {
+    if (++pc->mark <= 0) pc->mark = 1;
+}
+
 // Once per whole-signal call, after its channel ranges (`done`: all of them are queued).  A call pushes
 // ceil((len + taps - 1)/B) >= ceil(len/B) + P - 1 blocks, so the only spectrum of its input that can still be in the
 // delay line is in the slot the next block overwrites.  A recorded call has not run yet: it leaves `clear` alone.
@@ -996,11 +1133,12 @@ static ma_status close_whole(ma_pconv* pc, bool done) {
 
 // Whole-signal convolution of channels [c0, c0 + nc) (nc a multiple of the IR-sharing group): `in`
 // and `out` point at channel c0's rows.  Every buffer of the object is per channel, so a range runs
-// on its own slices; close_whole follows the last range.
+// on its own slices; open_whole comes before the first range, close_whole after the last.
 static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, int64_t len, int64_t in_stride,
                                float* out, int64_t out_stride, int64_t full) {
     ma_context* ctx = pc->ctx;
     const bool coarse = runs_coarse(pc);
+    const bool rescue = coarse && pc->w_plan != pc->plan;
     ma_fft_plan* plan = coarse ? pc->w_plan : pc->plan;
     const int B = coarse ? pc->w_block : pc->block, P = coarse ? pc->w_partitions : pc->partitions;
     const int64_t T = (full + B - 1) / B;
@@ -1032,6 +1170,8 @@ static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, in
         p.out_frame_stride = B;
         p.layout = LAYOUT_HALF_PACKED;
         p.mag_kind = MAG_NONE;
+        p.marks = rescue ? pc->d_marks + c0 : nullptr;
+        p.mark = pc->mark;
         MA_TRY(launch_r2c_small(plan, p));
     }
     // 3. delay-line multiply-accumulate for every (channel, block)
@@ -1056,6 +1196,17 @@ static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, in
         if (B >= 32 && P > 2 && T < (int64_t)1 << 30) MA_TRY(launch_mac_tiled(pc, q, nc, T, tl_len));
         else MA_TRY(launch_mac(pc, q, nc, false, T));
     }
+    // A call in place overwrites samples that pconv_rescue_kernel may want: their copy goes where the spectra were.
+    const float* samples = in;
+    int64_t samples_stride = in_stride;
+    const int64_t in_span = (nc - 1) * in_stride + len, out_span = (nc - 1) * out_stride + full;
+    if (rescue && in < out + out_span && out < in + in_span) {
+        float* copy = reinterpret_cast<float*>(timeline + (int64_t)(P - 1) * B);
+        MA_CUDA(cudaMemcpy2DAsync(copy, sizeof(float2) * (size_t)tl_stride, in, sizeof(float) * (size_t)(nc > 1 ? in_stride : len),
+                                  sizeof(float) * (size_t)len, (size_t)nc, cudaMemcpyDeviceToDevice, ctx->stream));
+        samples = copy;
+        samples_stride = 2 * tl_stride;
+    }
     // 4. inverse transform + block overlap-add, truncated at len + taps - 1
     {
         C2RParams p{};
@@ -1072,6 +1223,38 @@ static ma_status process_range(ma_pconv* pc, int c0, int nc, const float* in, in
         p.out_len = full;
         p.floor = -1.0f;
         MA_TRY(launch_istft_small(plan, p));
+    }
+    if (rescue) {
+        RescueParams p{};
+        p.in = samples;
+        p.len = len;
+        p.in_stride = samples_stride;
+        p.taps = pc->d_taps;
+        p.n_taps = pc->taps;
+        p.taps_stride = taps_stride(pc->taps);
+        p.ch2ir = pc->d_ch2ir + c0;
+        p.out = out;
+        p.out_stride = out_stride;
+        p.full = full;
+        p.marks = pc->d_marks + c0;
+        p.mark = pc->mark;
+        p.channels = nc;
+        p.block = pc->block;
+        p.coarse = B;
+        p.reach = (int64_t)pc->partitions * pc->block;
+        p.coarse_reach = (int64_t)P * B;
+        const int64_t chunks = (full + kRescueOutputs - 1) / kRescueOutputs, most = 4 * (int64_t)ctx->sm_count;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(chunks < most ? chunks : most));
+        cfg.blockDim = dim3(kRescueThreads);
+        cfg.stream = ctx->stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        (void)cudaLaunchKernelEx(&cfg, pconv_rescue_kernel, p);  // an error is picked up by after_launch
+        MA_TRY(after_launch(ctx));
     }
     // 5. the last P block spectra become the delay line (clear before the call: it stays clear, see close_whole)
     if (!coarse) {
@@ -1099,6 +1282,7 @@ ma_status ma_pconv_process_dev(ma_pconv* pc, const float* in, int64_t len, int64
     if (__builtin_add_overflow(len, pc->taps - 1, &full)) return MA_ERR_OUTPUT_OVERFLOW;
     if (len > pc->reserved_len) return MA_ERR_INVALID_ARGUMENT;
     if (pc->channels > 1 && (in_stride < len || out_stride < full)) return MA_ERR_INVALID_ARGUMENT;
+    open_whole(pc);
     const ma_status st = process_range(pc, 0, pc->channels, in, len, in_stride, out, out_stride, full);
     const ma_status closed = close_whole(pc, st == MA_OK);
     return st != MA_OK ? st : closed;
@@ -1125,6 +1309,7 @@ ma_status ma_pconv_process_host(ma_pconv* pc, const float* in, int64_t len, int6
     const int group = pc->share;  // channels that must stay together (they share one impulse response)
     const size_t in_row = round256(sizeof(float) * (size_t)len), out_row = round256(sizeof(float) * (size_t)full);
     const bool pinned = is_pinned(in) && is_pinned(out);
+    open_whole(pc);
     Pipe pp;
     MA_TRY(pipe_open(pp, ctx, pinned, C / group, (in_row + out_row) * (size_t)group, 0));
     const int64_t step = pp.chunk * group;

@@ -438,6 +438,47 @@ def test_taps_take_no_device_memory_before_a_reservation(lib, device):
     assert held <= need + (40 << 20)                           # the taps would be 64 MiB more
 
 
+@pytest.mark.parametrize("block,taps,length,where", [
+    (64, 3000, 9000, [(0, 4000)]), (64, 3000, 9000, [(0, 0)]), (64, 3000, 9000, [(1, 8999)]), (64, 3000, 9000, [(0, 255), (0, 256)]),
+    (32, 70000, 150001, [(0, 5), (0, 100000), (2, 149999)]), (256, 4096, 20000, [(1, 3), (1, 10001), (2, 511)]),
+    (1, 40, 3000, [(0, 100), (0, 1700)]), (2, 333, 5000, [(2, 2048)]), (128, 9000, 4097, [(0, 4096)]), (512, 40000, 70000, [(1, 33333)])])
+def test_non_finite_samples_spoil_the_callers_blocks_only(lib, device, block, taps, length, where):
+    """A NaN or infinity in the input of a call on the coarse partition: lost are exactly the outputs that the caller's
+    own block size loses, the others are the convolution's.  Also in place and through the host form."""
+    from metalaudio_b200 import Tensor
+    channels, full = 3, length + taps - 1
+    rng = np.random.default_rng(block + taps)
+    h = (rng.standard_normal((2, taps)) * np.exp(-np.arange(taps) / max(8, taps / 6))).astype(np.float32)
+    cmap = [0, 1, 1]
+    x = rng.standard_normal((channels, length)).astype(np.float32)
+    clean = x.copy()
+    for k, (c, at) in enumerate(where):
+        x[c, at] = (np.nan, np.inf, -np.inf)[k % 3]
+        clean[c, at] = 0.0
+    finite = np.ones((channels, full), bool)
+    for c, at in where:                      # block i of the output: input blocks i - P .. i
+        first = at // block * block
+        finite[c, first:first + (-(-taps // block) + 1) * block] = False
+    c = conv(device, block, channels=channels)
+    c.setKernel(h, channelToKernel=cmap)
+    zero_step(lib, device, c, block, channels)
+    assert np.array_equal(np.isfinite(c.process(x)), finite)      # the caller's block size
+    ref = np.stack([o64.convolve_full(clean[i], h[cmap[i]]) for i in range(channels)])
+
+    def check(y):
+        assert np.array_equal(np.isfinite(y), finite)
+        for i in range(channels):
+            assert o64.rel_rms(y[i][finite[i]], ref[i][finite[i]]) <= TOL
+    check(c.process(x))
+    buf = Tensor(device, (channels, full))
+    buf.copy(np.pad(x, ((0, 0), (0, taps - 1))))
+    assert lib.ma_pconv_process_dev(c._h, ctypes.c_void_p(buf.pointer), length, full, ctypes.c_void_p(buf.pointer), full) == 0
+    device.synchronize(30)
+    check(buf.toArray())
+    y = c.process(clean)                       # nothing is left behind
+    assert all(o64.rel_rms(y[i], ref[i]) <= TOL for i in range(channels))
+
+
 class Recorded:
     """Calls on the library's stream recorded into a CUDA graph."""
 
