@@ -253,101 +253,74 @@ static ma_status launch_istft_rows(ma_fft_plan* plan, const C2RParams& p, size_t
     return after_launch(ctx);
 }
 
+// The fast kernels (see istft_fast_body).  Contiguous ranges of the global frame list, one wave of them: a range pays
+// for `reach` lead-in frames, yet the wave lasts as long as one range, so fewer, longer ranges only leave SMs idle
+// (8 signals of 332 frames, 4096 points, hop 1024: 55 ranges of 48 frames 110 us, 532 of 5 frames 69 us).
+template <int M, int LAYOUT, int OVT, bool PLAIN = false, bool EXACT = PLAIN>
+static ma_status launch_istft_fast(ma_fft_plan* plan, const C2RParams& p) {
+    constexpr int T = FftPlan<M>::T;
+    constexpr size_t smem = (size_t)IstftFastShape<M, OVT, PLAIN>::SMEM_BYTES;
+    static int per_sm[64] = {0};
+    ma_context* ctx = plan->ctx;
+    int& occ = per_sm[ctx->device & 63];
+    if (occ == 0) MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT, OVT, PLAIN, EXACT>, T, smem, &occ));
+    const int64_t total = p.frames_per_signal * p.n_signals, cap = (int64_t)ctx->sm_count * occ;
+    istft_fast_kernel<M, LAYOUT, OVT, PLAIN, EXACT><<<(unsigned)(total < cap ? total : cap), T, smem, ctx->stream>>>(p);
+    return after_launch(ctx);
+}
+
 template <int M>
 static ma_status launch_istft_t(ma_fft_plan* plan, C2RParams& p) {
     constexpr int T = FftPlan<M>::T;
     const bool fast = istft_fast_ok<M>(p);
+    if constexpr (plan_pairable<M>()) {
+        if (fast && istft_plain<M>(p)) return launch_istft_fast<M, LAYOUT_HALF_PACKED, 2, true>(plan, p);
+    }
     if constexpr (CtaShape<M>::FPC >= kRowsFromSlots) {
         const size_t rows_smem = istft_rows_smem<M>(p.hop);
         // The fast kernel's CTA is one frame's threads: less than a warp below 1024 points (256 points, hop 64: STFT and
-        // iSTFT of 256 x 300000 samples 1800 us with it, 1423 us with the rows).  The plain overlap-add of
-        // convolution blocks, which stages packed rows, is the faster one at any length.
-        if ((!fast || (T < 32 && !istft_plain<M>(p))) && rows_smem <= kRowsSmemLimit) {
+        // iSTFT of 256 x 300000 samples 1800 us with it, 1423 us with the rows).  Only the plain overlap-add of
+        // convolution blocks, which stages packed rows, is the faster one at any length.  Hops that the fast kernel
+        // could serve there leave few enough rows for the limit (31 of 256 samples).
+        if ((!fast || T < 32) && rows_smem <= kRowsSmemLimit) {
             return p.layout == LAYOUT_HALF_INTERLEAVED
                        ? launch_istft_rows<M, LAYOUT_HALF_INTERLEAVED>(plan, p, rows_smem, &plan->rows_occ[0])
                        : launch_istft_rows<M, -1>(plan, p, rows_smem, &plan->rows_occ[1]);
         }
     }
-    const int ov = fast ? (2 * M) / p.hop : 0;
-    // 0: general kernel; 1: fast, overlap count read at run time; 2: fast with the overlap count 4
-    // fixed at compile time (register ring); 3: the convolution's block overlap-add; 4: overlap count 2;
-    // 5: a hop that does not divide the frame
-    const int kind = !fast ? 0 : istft_plain<M>(p) ? 3 : ov == 2 && 2 * p.hop == 2 * M && p.layout == LAYOUT_HALF_INTERLEAVED ? 4
-                   : (ov == 4 && 4 * p.hop == 2 * M) ? 2 : (2 * M) % p.hop != 0 ? 5 : 1;
-    const size_t smem = kind == 4 ? (size_t)IstftFastShape<M, 2>::SMEM_BYTES
-                      : kind == 3 ? (size_t)IstftFastShape<M, 2, true>::SMEM_BYTES
-                      : kind == 2 ? (size_t)IstftFastShape<M, 4>::SMEM_BYTES
-                      : kind == 1 || kind == 5 ? (size_t)IstftFastShape<M, 0>::SMEM_BYTES
-                                  : 2 * smem_elems_per_fft<M, 1>() * sizeof(float2) + 2 * M * sizeof(float);
-    static int per_sm[6][64] = {{0}, {0}, {0}, {0}, {0}, {0}};
-    ma_context* ctx = plan->ctx;
-    int& occ = per_sm[kind][ctx->device & 63];
-    const int variant = !fast || kind >= 3 ? 0
-                              : (p.layout == LAYOUT_HALF_INTERLEAVED ? 1 : (p.layout == LAYOUT_HALF_PACKED ? 3 : 5)) +
-                                    (kind == 2 ? 1 : 0);
-    if (occ == 0) {  // the layout variants of a kind share its footprint; raise every one's shared-memory limit
-        int dummy;
-        if (kind == 5) {
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0, false, true>, T, smem, &occ));
-        } else if (kind == 4) {
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 2>, T, smem, &occ));
-        } else if (kind == 3) {
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true>, T, smem, &occ));
-        } else if (kind == 2) {
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 4>, T, smem, &occ));
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 4>, T, smem, &dummy));
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_POLAR, 4>, T, smem, &dummy));
-        } else if (kind == 1) {
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0>, T, smem, &occ));
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_PACKED, 0>, T, smem, &dummy));
-            MA_TRY(occupancy(istft_fast_kernel<M, LAYOUT_HALF_POLAR, 0>, T, smem, &dummy));
-        } else {
-            MA_TRY(occupancy(istft_kernel<M>, T, smem, &occ));
+    if constexpr (plan_pairable<M>() && T >= 32) {
+        // Overlap counts of 4 and, in the interleaved layout, 2 are fixed at compile time (register ring); hops that
+        // do not divide the frame come in the interleaved layout only (istft_fast_ok).
+        if (fast && 4 * p.hop == 2 * M) {
+            if (p.layout == LAYOUT_HALF_INTERLEAVED) return launch_istft_fast<M, LAYOUT_HALF_INTERLEAVED, 4>(plan, p);
+            if (p.layout == LAYOUT_HALF_PACKED) return launch_istft_fast<M, LAYOUT_HALF_PACKED, 4>(plan, p);
+            return launch_istft_fast<M, LAYOUT_HALF_POLAR, 4>(plan, p);
+        }
+        if (fast) {
+            if (p.layout == LAYOUT_HALF_PACKED) return launch_istft_fast<M, LAYOUT_HALF_PACKED, 0>(plan, p);
+            if (p.layout == LAYOUT_HALF_POLAR) return launch_istft_fast<M, LAYOUT_HALF_POLAR, 0>(plan, p);
+            if (p.hop == M) return launch_istft_fast<M, LAYOUT_HALF_INTERLEAVED, 2>(plan, p);
+            if ((2 * M) % p.hop != 0) return launch_istft_fast<M, LAYOUT_HALF_INTERLEAVED, 0, false, true>(plan, p);
+            return launch_istft_fast<M, LAYOUT_HALF_INTERLEAVED, 0>(plan, p);
         }
     }
-    const int64_t F = p.frames_per_signal;
-    const int64_t cap = (int64_t)ctx->sm_count * occ;
-    int64_t total;
-    if (fast) {
-        // Contiguous ranges of the global frame list, one wave of them.  A range pays for `reach` lead-in frames,
-        // yet the wave lasts as long as one range: fewer, longer ranges only leave SMs idle (8 signals of
-        // 332 frames, 4096 points, hop 1024: 55 ranges of 48 frames 110 us, 532 of 5 frames 69 us).
-        total = F * p.n_signals;
-    } else {
-        // Chunks per signal: two waves of CTAs where the lead-in frames stay a small fraction of a chunk, at least
-        // one wave in any case.
-        const int reach = (2 * M + p.hop - 1) / p.hop - 1;
-        const int64_t min_len = reach > 0 ? 16 * (int64_t)reach : 1;
-        int64_t chunks = (2 * cap + p.n_signals - 1) / p.n_signals;
-        if (chunks > F / min_len) chunks = F / min_len;
-        if (chunks < cap / p.n_signals) chunks = cap / p.n_signals < F ? cap / p.n_signals : F;
-        if (chunks < 1) chunks = 1;
-        p.chunks_per_signal = (int32_t)chunks;
-        total = chunks * p.n_signals;
-    }
-    const int grid = (int)(total < cap ? total : cap);
-    if (grid < 1) return MA_OK;
-    if (kind == 3) {
-        istft_fast_kernel<M, LAYOUT_HALF_PACKED, 2, true><<<grid, T, smem, ctx->stream>>>(p);
-        return after_launch(ctx);
-    }
-    if (kind == 5) {
-        istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0, false, true><<<grid, T, smem, ctx->stream>>>(p);
-        return after_launch(ctx);
-    }
-    if (kind == 4) {
-        istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 2><<<grid, T, smem, ctx->stream>>>(p);
-        return after_launch(ctx);
-    }
-    switch (variant) {
-        case 1: istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 0><<<grid, T, smem, ctx->stream>>>(p); break;
-        case 2: istft_fast_kernel<M, LAYOUT_HALF_INTERLEAVED, 4><<<grid, T, smem, ctx->stream>>>(p); break;
-        case 3: istft_fast_kernel<M, LAYOUT_HALF_PACKED, 0><<<grid, T, smem, ctx->stream>>>(p); break;
-        case 4: istft_fast_kernel<M, LAYOUT_HALF_PACKED, 4><<<grid, T, smem, ctx->stream>>>(p); break;
-        case 5: istft_fast_kernel<M, LAYOUT_HALF_POLAR, 0><<<grid, T, smem, ctx->stream>>>(p); break;
-        case 6: istft_fast_kernel<M, LAYOUT_HALF_POLAR, 4><<<grid, T, smem, ctx->stream>>>(p); break;
-        default: istft_kernel<M><<<grid, T, smem, ctx->stream>>>(p); break;
-    }
+    constexpr size_t smem = 2 * smem_elems_per_fft<M, 1>() * sizeof(float2) + 2 * M * sizeof(float);
+    static int per_sm[64] = {0};
+    ma_context* ctx = plan->ctx;
+    int& occ = per_sm[ctx->device & 63];
+    if (occ == 0) MA_TRY(occupancy(istft_kernel<M>, T, smem, &occ));
+    // Chunks per signal: two waves of CTAs where the lead-in frames stay a small fraction of a chunk, at least
+    // one wave in any case.
+    const int64_t F = p.frames_per_signal, cap = (int64_t)ctx->sm_count * occ;
+    const int reach = (2 * M + p.hop - 1) / p.hop - 1;
+    const int64_t min_len = reach > 0 ? 16 * (int64_t)reach : 1;
+    int64_t chunks = (2 * cap + p.n_signals - 1) / p.n_signals;
+    if (chunks > F / min_len) chunks = F / min_len;
+    if (chunks < cap / p.n_signals) chunks = cap / p.n_signals < F ? cap / p.n_signals : F;
+    if (chunks < 1) chunks = 1;
+    p.chunks_per_signal = (int32_t)chunks;
+    const int64_t total = chunks * p.n_signals;
+    istft_kernel<M><<<(unsigned)(total < cap ? total : cap), T, smem, ctx->stream>>>(p);
     return after_launch(ctx);
 }
 
