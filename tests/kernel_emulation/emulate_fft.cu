@@ -107,12 +107,14 @@ int emul_istft(int n, int hop, const float* in_a, const float* in_b, long long i
     {                                                                                            \
         constexpr int ELEMS = smem_elems_per_fft<MM, 1>();                                       \
         const bool fast = istft_fast_ok<MM>(p);                                                  \
-        const size_t smem = fast ? (size_t)(2 * MM / hop == 4 ? IstftFastShape<MM, 4>::SMEM_BYTES : IstftFastShape<MM, 0>::SMEM_BYTES) \
+        const size_t smem = fast ? (size_t)(4 * hop == n ? IstftFastShape<MM, 4>::SMEM_BYTES     \
+                                            : 2 * hop == n ? IstftFastShape<MM, 2>::SMEM_BYTES : IstftFastShape<MM, 0>::SMEM_BYTES) \
                                  : 2 * ELEMS * sizeof(float2) + (size_t)n * sizeof(float);       \
         used_fast = fast ? 1 : 0;                                                                \
         run_grid(nblocks, FftPlan<MM>::T, smem, [&](HostCta& cta, void* sm) {                    \
             if constexpr (plan_pairable<MM>()) {                                                 \
-                if (fast && 2 * MM / hop == 4) { istft_fast_body<MM, 0, 4, HostCta>(p, cta, (float2*)sm); return; } \
+                if (fast && 4 * hop == n) { istft_fast_body<MM, 0, 4, HostCta>(p, cta, (float2*)sm); return; } \
+                if (fast && 2 * hop == n) { istft_fast_body<MM, 0, 2, HostCta>(p, cta, (float2*)sm); return; } \
                 if (fast && n % hop != 0) { istft_fast_body<MM, 0, 0, HostCta, false, true>(p, cta, (float2*)sm); return; } \
                 if (fast) { istft_fast_body<MM, 0, 0, HostCta>(p, cta, (float2*)sm); return; }   \
             }                                                                                    \

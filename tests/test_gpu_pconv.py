@@ -291,9 +291,9 @@ def _c4_case(channels=4, extra_blocks=256):
 
 
 def test_config4_true_partition_count_whole_signal(device):
-    """Configuration 4 at its real partition count (block 64, 262144 taps, 4096 partitions, one
-    impulse response per channel pair): the whole-signal call sums 4096 products per output bin in
-    float32; against the float64 linear convolution and the float32 port of the reference loop."""
+    """Configuration 4's block size and taps (block 64, 262144 taps, one impulse response per channel pair), a
+    whole-signal call on a clear delay line: it runs on 64 partitions of 4096 samples.  Against the float64 linear
+    convolution and the float32 port of the reference loop, which sums 4096 products per output bin."""
     irs, x, ref = _c4_case()
     c = conv(device, C4_BLOCK, channels=4)
     c.setKernel(irs, channelToKernel=[0, 0, 1, 1])
@@ -312,6 +312,28 @@ def test_config4_true_partition_count_whole_signal(device):
     yp = port.process(short)
     ys = c.process(np.stack([short] * 4))[0]
     assert o64.rel_rms(ys, yp) <= TOL
+
+
+@pytest.mark.parametrize("partitions", [2047, 2048, 4096])
+def test_whole_signal_sums_of_thousands_of_partitions(device, lib, partitions):
+    """Whole-signal calls that continue a stream keep the caller's partition: up to 4096 products of block 64 per output
+    bin, from 2048 partitions up as sums of at most 256 that are added up in a second level.  Inputs reach past the
+    ramp-up, so that every partition meets a non-zero spectrum."""
+    taps = partitions * C4_BLOCK - 5
+    irs = configs.c4_irs(n_irs=2, taps=taps)
+    x = configs.c4_input(channels=2, length=(partitions + 130) * C4_BLOCK + 13)
+    ref = np.stack([o64.convolve_full(x[i], irs[i]) for i in range(2)])
+    c = conv(device, C4_BLOCK, channels=2)
+    c.setKernel(irs, channelToKernel=[0, 1])
+    assert c.partitionCount == partitions
+    zero_step(lib, device, c, C4_BLOCK, 2)
+    y = c.process(x)
+    # float32 sums of n terms err by about 2^-24 sqrt(n): 256 terms 9.5e-7, 2047 terms 2.7e-6
+    bound = 1e-6 if partitions >= 2048 else 2.7e-6
+    assert o64.rel_rms(y, ref) <= bound
+    lo, hi = taps, x.shape[1]
+    assert o64.rel_rms(y[:, lo:hi], ref[:, lo:hi]) <= bound
+    print("partitions", partitions, o64.rel_rms(y, ref), o64.rel_rms(y[:, lo:hi], ref[:, lo:hi]), o64.max_over_rms(y, ref))
 
 
 def test_config4_true_partition_count_streaming(device, lib):

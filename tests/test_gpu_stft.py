@@ -55,6 +55,42 @@ def test_stft_istft_parity(device, n, hop, length, kind):
     assert np.all(np.abs(y - yref) <= 1e-5 * np.sqrt(n) / np.sqrt(ws) + 1e-5)
 
 
+# The batched half-spectrum calls have kernels of their own by hop: a quarter and a half of the frame (register
+# rings), other multiples of the threads' span that divide the frame or not (thread-private ring), the rest, and short
+# frames side by side in a CTA; lengths are odd where signals then start on odd samples.
+BATCHED = [(8192, 4096, 40001, 5), (8192, 2048, 40960, 3), (8192, 2560, 50003, 2), (8192, 1024, 30000, 2), (8192, 8192, 60000, 2),
+           (4096, 2048, 30001, 7), (4096, 1280, 30000, 3), (4096, 512, 20001, 2), (4096, 3072, 40000, 2), (4096, 1365, 20000, 2),
+           (2048, 1024, 9001, 3), (2048, 640, 9000, 4), (1024, 512, 5000, 9), (1024, 320, 5001, 4), (512, 256, 4000, 5),
+           (512, 160, 4001, 20), (256, 128, 3000, 4), (256, 80, 2999, 33), (256, 64, 3000, 3), (64, 32, 700, 40), (64, 20, 701, 3),
+           (4096, 2048, 4096, 3), (8192, 4096, 12288, 1), (1024, 320, 1024, 2)]
+
+
+@pytest.mark.parametrize("n,hop,length,signals", BATCHED)
+def test_batched_half_spectra(device, n, hop, length, signals):
+    """stftBatch with and without magnitudes and istftBatch, interleaved half spectra, against float64: the interior, the
+    ends (rounding amplified by 1/sum(w^2)), and runs that repeat bit for bit."""
+    from metalaudio_b200 import FFT
+    x = np.random.default_rng(n + 3 * hop).uniform(-1, 1, (signals, length)).astype(np.float32)
+    w = rp.periodic_hann(n)
+    fft = FFT(device, FFT.Config(size=n, hopSize=hop), window=w)
+    ref = o64.stft(x, n, hop, w)
+    spec, mag = fft.stftBatch(x, magnitude=True)
+    assert o64.rel_rms(spec, ref) <= 1e-6
+    assert o64.rel_rms(mag, np.abs(ref)) <= 1e-6
+    assert o64.rel_rms(fft.stftBatch(x), ref) <= 1e-6
+    y = fft.istftBatch(spec)
+    frames = ref.shape[1]
+    floor = float(rp.window_floor())
+    yref = o64.istft(ref, n, hop, w, floor)
+    assert y.shape == yref.shape
+    m = interior(frames, n, hop, w)
+    # 1e-6 for sums of unit weight; where hops are wide the window sum dips to 1e-2 of its maximum, which divides the error
+    assert o64.rel_rms(y[:, m], yref[:, m]) <= TOL
+    ws = np.maximum(rp.window_sum(frames, n, hop, w, floor), floor)
+    assert np.all(np.abs(y - yref) <= 1e-5 * np.sqrt(n) / np.sqrt(ws) + 1e-5)
+    assert np.array_equal(fft.istftBatch(spec), y)
+
+
 def test_stft_input_too_short(device):
     from metalaudio_b200 import FFT, FFTError
     fft = FFT(device, FFT.Config(size=256))

@@ -97,7 +97,11 @@ def test_zero_padded_frames(emul):
                                                       (1024, 1024, 8192, 2, "none"), (8, 2, 50, 2, "hann"),
                                                       (4, 1, 20, 1, "hann"), (2, 1, 9, 2, "none"),
                                                       (4096, 1024, 30000, 2, "hann"), (4096, 256, 12000, 1, "hann"),
-                                                      (2048, 1024, 9000, 3, "hamming"), (64, 8, 300, 1, "hann")])
+                                                      (2048, 1024, 9000, 3, "hamming"), (64, 8, 300, 1, "hann"),
+                                                      # hops of half a frame (register ring of two) and non-dividing ones
+                                                      (4096, 2048, 13001, 1, "hann"), (8192, 4096, 30000, 2, "hann"),
+                                                      (2048, 1024, 2048, 1, "hann"), (2048, 1024, 3072, 1, "hann"),
+                                                      (4096, 1280, 16000, 1, "hann"), (8192, 2560, 30000, 1, "hamming")])
 def test_stft_istft(emul, n, hop, length, chunks, kind):
     m = n // 2
     w = rp.window(kind, n)
