@@ -67,7 +67,6 @@ bool is_pinned(const void* p) {
 // Pageable arrays cross the staging buffer in pieces.  A piece's memcpy (first touch of fresh pages above all)
 // takes several times its transfer, so arrays of 2 MiB and more are copied by up to four threads: each
 // takes every fourth piece, and transfers run while other pieces are copied.  The threads end with the call.
-constexpr size_t kThreadedCopyFrom = (size_t)2 << 20;
 static_assert(kCopyPieces % kCopyThreads == 0, "pieces are dealt out evenly");
 
 static int copy_threads() {

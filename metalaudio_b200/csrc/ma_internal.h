@@ -9,7 +9,9 @@
 #include "../../include/metalaudio_cuda.h"
 
 constexpr int kAuxStreams = 3;
-constexpr int kCopyPieces = 16, kCopyThreads = 4;  // threaded copies of pageable arrays (context.cu)
+// Copies of pageable arrays by several threads (context.cu).
+constexpr int kCopyPieces = 16, kCopyThreads = 4;
+constexpr size_t kThreadedCopyFrom = (size_t)2 << 20;
 
 struct ma_context {
     int device = 0;

@@ -15,11 +15,14 @@
 #include <cuda_pipeline.h>
 
 #include <atomic>
+#include <cstring>
+#include <memory>
 #include <new>
 #include <type_traits>
 #include <vector>
 
 #include "bulk_copy.cuh"
+#include "copy_threads.h"
 #include "fft_plan.h"
 #include "host_pipe.h"
 #include "pconv_tiling.h"
@@ -47,7 +50,7 @@ struct ma_pconv {
     // Whole-signal calls that start on a clear delay line need not keep the caller's block size: they run on
     // a coarser partition of the same taps (whole_block), built by ma_pconv_reserve.  Where the caller's own
     // block is the better one, or the only one there is memory for, w_plan and d_hw are plan and d_h.
-    std::vector<float> h_taps;    // [n_irs][taps], from set_kernels until the coarse spectra and their buffers exist
+    std::unique_ptr<float[]> h_taps;  // [n_irs][taps_stride], from set_kernels until the coarse spectra and their buffers exist
     float* d_taps = nullptr;      // [n_irs][taps_stride], beside the coarse spectra (pconv_rescue_kernel)
     int32_t* d_marks = nullptr;   // [channels]: the call that last met a non-finite sample in the channel
     int32_t mark = 0;             // number of the latest coarse call
@@ -674,10 +677,12 @@ static ma_status partition_spectra(ma_pconv* pc, ma_fft_plan* plan, const float*
     return launch_r2c_small(plan, p);
 }
 
-// The taps on the device, rows taps_stride apart.
+// The taps on the device, rows taps_stride apart: the host copy as one transfer, or the caller's rows.
 static ma_status upload_taps(ma_pconv* pc, const float* irs, float* d_taps) {
+    const int64_t stride = taps_stride(pc->taps);
+    if (pc->h_taps != nullptr) return copy_h2d(pc->ctx, d_taps, pc->h_taps.get(), sizeof(float) * (size_t)(stride * pc->n_irs));
     for (int i = 0; i < pc->n_irs; ++i)
-        MA_TRY(copy_h2d(pc->ctx, d_taps + (int64_t)i * taps_stride(pc->taps), irs + (int64_t)i * pc->taps, sizeof(float) * (size_t)pc->taps));
+        MA_TRY(copy_h2d(pc->ctx, d_taps + i * stride, irs + i * pc->taps, sizeof(float) * (size_t)pc->taps));
     return MA_OK;
 }
 
@@ -843,7 +848,7 @@ static ma_status build_coarse(ma_pconv* pc) {
     ma_context* ctx = pc->ctx;
     pc->w_block = whole_block(pc->block, pc->taps);
     pc->w_partitions = (int)((pc->taps + pc->w_block - 1) / pc->w_block);
-    if (pc->w_block == pc->block || pc->h_taps.empty()) {
+    if (pc->w_block == pc->block || pc->h_taps == nullptr) {
         use_own_block(pc);
         return MA_OK;
     }
@@ -856,7 +861,7 @@ static ma_status build_coarse(ma_pconv* pc) {
         if (e == cudaSuccess) e = cudaMemsetAsync(pc->d_marks, 0, sizeof(int32_t) * (size_t)pc->channels, ctx->stream);
         if (e != cudaSuccess) st = cuda_fail(e);
     }
-    if (st == MA_OK) st = upload_taps(pc, pc->h_taps.data(), pc->d_taps);
+    if (st == MA_OK) st = upload_taps(pc, nullptr, pc->d_taps);
     if (st == MA_OK) st = partition_spectra(pc, pc->w_plan, pc->d_taps, pc->w_block, pc->w_partitions, pc->d_hw);
     if (st == MA_OK) {
         const cudaError_t e = cudaStreamSynchronize(ctx->stream);
@@ -894,9 +899,31 @@ static ma_status alloc_signal_buffers(ma_pconv* pc, int64_t full) {
     return st;
 }
 
+// The host copy that ma_pconv_reserve lays out in coarse blocks; without the memory for it whole-signal calls keep the
+// caller's block size.  Fresh pages make one thread's copy slow: four share it from 2 MiB up, and
+// it makes the uploads one transfer (128 responses of 65536 taps: setting them 5.4 -> 6.4 ms, 8.6 with one thread and
+// a transfer per row; with the reservation 7 -> 10.5 ms, 16 that way).
+static void keep_taps(ma_pconv* pc, const float* irs) {
+    const int64_t taps = pc->taps, stride = taps_stride(taps), count = taps * pc->n_irs;
+    pc->h_taps.reset(new (std::nothrow) float[(size_t)(stride * pc->n_irs)]);
+    float* const to = pc->h_taps.get();
+    if (to == nullptr) return;
+    auto part = [&](int64_t at, int64_t end) {
+        while (at < end) {
+            const int64_t row = at / taps, off = at - row * taps, n = end - at < taps - off ? end - at : taps - off;
+            std::memcpy(to + row * stride + off, irs + at, sizeof(float) * (size_t)n);
+            at += n;
+        }
+    };
+    if (sizeof(float) * (size_t)count < kThreadedCopyFrom) part(0, count);
+    else on_threads<kCopyThreads>([&](int i) { part(count / kCopyThreads * i, i + 1 < kCopyThreads ? count / kCopyThreads * (i + 1) : count); });
+    for (int64_t row = 0; row < pc->n_irs; ++row)
+        for (int64_t k = taps; k < stride; ++k) to[row * stride + k] = 0.f;
+}
+
 static void free_kernel_buffers(ma_pconv* pc) {
     free_coarse(pc);
-    pc->h_taps = std::vector<float>();
+    pc->h_taps.reset();
     if (pc->d_h) (void)cudaFree(pc->d_h);
     if (pc->d_ch2ir) (void)cudaFree(pc->d_ch2ir);
     if (pc->d_ring) (void)cudaFree(pc->d_ring);
@@ -1019,16 +1046,11 @@ ma_status ma_pconv_set_kernels(ma_pconv* pc, const float* irs, int64_t taps, int
     if (e != cudaSuccess) st = cuda_fail(e);
     if (st == MA_OK) st = copy_h2d(ctx, pc->d_ch2ir, map.data(), sizeof(int32_t) * (size_t)C);
     float* d_taps = nullptr;
+    if (st == MA_OK && whole_block(B, taps) != B) keep_taps(pc, irs);
     if (st == MA_OK) st = temp_alloc(ctx, sizeof(float) * (size_t)(taps_stride(taps) * n_irs), (void**)&d_taps);
     if (st == MA_OK) st = upload_taps(pc, irs, d_taps);
     if (st == MA_OK) st = partition_spectra(pc, pc->plan, d_taps, B, P, pc->d_h);
     temp_free(ctx, d_taps);
-    if (st == MA_OK && whole_block(B, taps) != B) {
-        try {
-            pc->h_taps.assign(irs, irs + taps * n_irs);
-        } catch (const std::bad_alloc&) {  // whole-signal calls keep the caller's block size
-        }
-    }
     if (st == MA_OK) st = ma_pconv_reset(pc);
     if (st == MA_OK) {
         cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
@@ -1099,7 +1121,7 @@ ma_status ma_pconv_reserve(ma_pconv* pc, int64_t max_len) {
         free_coarse(pc);  // the next call lays the taps out afresh
         return st;
     }
-    pc->h_taps = std::vector<float>();
+    pc->h_taps.reset();
     pc->reserved_len = max_len;
     return MA_OK;
 }
